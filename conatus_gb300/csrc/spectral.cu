@@ -30,7 +30,9 @@
 
 #include "common.cuh"
 #include "conatus_gb300.h"
+#include "expand.cuh"
 #include "fft.cuh"
+#include "fixed_transforms.cuh"
 
 namespace cng {
 
@@ -244,41 +246,6 @@ __global__ void k_cheb_fwd_grp(const __grid_constant__ Grp<ChebArgs<R>> g) {
     const int k = g.find(blockIdx.x);
     const ChebArgs<R>& a = g.a[k];
     cheb_fwd_body<R>(blockIdx.x - g.start[k], a.in, a.out, a.ncols, a.N, a.plan, a.B, a.tw, a.tq);
-}
-
-// ------------------------------------------------------------------------------------------------
-// Derivative expansion fused into the load of a backward transform (fields that differ only by a
-// derivative along the transform's axis share the transforms before it): output group og of the
-// batch reads input group src[og] and multiplies each value by (i k_j)^ord[og], k_j the wavenumber
-// of its index j along the axis, from a table [order - 1][nidx] rounded to R on the host. Outer row
-// o = (c nout + og) per + r reads row (c nin + src[og]) per + r.
-template <class R>
-struct Expand {
-    int nout = 0;                 // 0: no expansion (row o reads row o)
-    int nin = 0, per = 1, nidx = 0;
-    const int* src = nullptr;
-    const int* ord = nullptr;
-    const c2<R>* tab = nullptr;
-};
-
-// the source row of outer row o and its factor table (nullptr: no derivative)
-template <class R>
-__device__ __forceinline__ long long expand_row(const Expand<R>& ex, long long o, const c2<R>** wt) {
-    *wt = nullptr;
-    if (ex.nout == 0) return o;
-    const long long g = o / ex.per;
-    const long long r = o - g * ex.per;
-    const long long c = g / ex.nout;
-    const int og = (int)(g - c * ex.nout);
-    const int od = ex.ord[og];
-    if (od > 0) *wt = ex.tab + (size_t)(od - 1) * ex.nidx;
-    return (c * ex.nin + ex.src[og]) * ex.per + r;
-}
-
-// w v with w = (i k)^o (the product of the separate expansion pass)
-template <class R>
-__device__ __forceinline__ c2<R> ikmul(c2<R> w, c2<R> v) {
-    return mk<R>(w.x * v.x - w.y * v.y, w.x * v.y + w.y * v.x);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -962,46 +929,62 @@ static Planned<AxisArgs<R>> plan_axis(bool real, const void* in, void* out, long
     return p;
 }
 
+// FP64: the fixed-point transforms (fixed_transforms.cu), or `fp64` ones for problems without a Fourier
+// direction. Those have a column per field, which gains nothing (Burgers N = 128: 9.4 against 9.9 us,
+// all latency), and their tau systems (condition ~ N^4, one system) hand each rounding of F on some
+// 1e5 times larger: they keep the roundings they have.
 template <class R>
 void launch_cheb(const c2<R>* in, c2<R>* out, long long ncols, int N, int M, bool forward, cudaStream_t st,
-                 int maxseq = 0, int threads = 0) {
-    if (threads <= 0) threads = kFftThreads;
+                 int maxseq = 0, int threads = 0, bool fp64 = false) {
     if (ncols <= 0) return;
     if (N == 1 && M == 1) {        // no Chebyshev direction: the single coefficient is the value
         CNG_CUDA(cudaMemcpyAsync(out, in, sizeof(c2<R>) * (size_t)ncols, cudaMemcpyDeviceToDevice, st));
         return;
     }
-    set_smem_attr<R>((const void*)k_cheb_bwd<R>);
-    set_smem_attr<R>((const void*)k_cheb_fwd<R>);
-    const auto p = plan_cheb<R>(in, out, ncols, N, M, forward, maxseq);
-    const ChebArgs<R>& a = p.a;
-    if (forward) k_cheb_fwd<R><<<p.blocks, threads, p.smem, st>>>(a.in, a.out, a.ncols, a.N, a.plan, a.B, a.tw, a.tq);
-    else k_cheb_bwd<R><<<p.blocks, threads, p.smem, st>>>(a.in, a.out, a.ncols, a.N, a.plan, a.B, a.tw, a.tq);
-    CNG_LAUNCH("k_cheb");
+    if (sizeof(R) == 8 && !fp64) {
+        if constexpr (sizeof(R) == 8) fx_cheb({FxChebJob{in, out, ncols, N, M, maxseq}}, forward, st, threads);
+    } else {
+        if (threads <= 0) threads = kFftThreads;
+        set_smem_attr<R>((const void*)k_cheb_bwd<R>);
+        set_smem_attr<R>((const void*)k_cheb_fwd<R>);
+        const auto p = plan_cheb<R>(in, out, ncols, N, M, forward, maxseq);
+        const ChebArgs<R>& a = p.a;
+        if (forward) k_cheb_fwd<R><<<p.blocks, threads, p.smem, st>>>(a.in, a.out, a.ncols, a.N, a.plan, a.B, a.tw, a.tq);
+        else k_cheb_bwd<R><<<p.blocks, threads, p.smem, st>>>(a.in, a.out, a.ncols, a.N, a.plan, a.B, a.tw, a.tq);
+        CNG_LAUNCH("k_cheb");
+    }
 }
 
 template <class R>
 void launch_fft_axis(const c2<R>* in, c2<R>* out, long long outer, int inner, int Nc, int L, bool forward,
                      cudaStream_t st, int maxseq = 0, int threads = 0, Expand<R> ex = Expand<R>{}) {
-    if (threads <= 0) threads = kFftThreads;
     if (outer <= 0 || inner <= 0) return;
-    set_smem_attr<R>((const void*)k_fft_axis<R>);
-    const auto p = plan_axis<R>(false, in, out, outer, inner, Nc, L, forward, maxseq, ex);
-    k_fft_axis<R><<<p.blocks, threads, p.smem, st>>>(in, out, outer, inner, Nc, p.a.plan, p.a.B, p.a.forward,
-                                                      p.a.tw, ex);
-    CNG_LAUNCH("k_fft_axis");
+    if constexpr (sizeof(R) == 8) {
+        fx_axis({FxAxisJob{in, out, outer, inner, Nc, L, maxseq, ex}}, false, forward, st, threads);
+    } else {
+        if (threads <= 0) threads = kFftThreads;
+        set_smem_attr<R>((const void*)k_fft_axis<R>);
+        const auto p = plan_axis<R>(false, in, out, outer, inner, Nc, L, forward, maxseq, ex);
+        k_fft_axis<R><<<p.blocks, threads, p.smem, st>>>(in, out, outer, inner, Nc, p.a.plan, p.a.B, p.a.forward,
+                                                          p.a.tw, ex);
+        CNG_LAUNCH("k_fft_axis");
+    }
 }
 
 template <class R>
 void launch_rfft_axis(const void* in, void* out, long long outer, int inner, int K, int L, bool forward,
                       cudaStream_t st, int maxseq = 0, int threads = 0, Expand<R> ex = Expand<R>{}) {
-    if (threads <= 0) threads = kFftThreads;
     if (outer <= 0 || inner <= 0) return;
-    set_smem_attr<R>((const void*)k_rfft_axis<R>);
-    const auto p = plan_axis<R>(true, in, out, outer, inner, K, L, forward, maxseq, ex);
-    k_rfft_axis<R><<<p.blocks, threads, p.smem, st>>>(in, out, outer, inner, K, p.a.plan, p.a.B, p.a.forward,
-                                                       p.a.tw, ex);
-    CNG_LAUNCH("k_rfft_axis");
+    if constexpr (sizeof(R) == 8) {
+        fx_axis({FxAxisJob{in, out, outer, inner, K, L, maxseq, ex}}, true, forward, st, threads);
+    } else {
+        if (threads <= 0) threads = kFftThreads;
+        set_smem_attr<R>((const void*)k_rfft_axis<R>);
+        const auto p = plan_axis<R>(true, in, out, outer, inner, K, L, forward, maxseq, ex);
+        k_rfft_axis<R><<<p.blocks, threads, p.smem, st>>>(in, out, outer, inner, K, p.a.plan, p.a.B, p.a.forward,
+                                                           p.a.tw, ex);
+        CNG_LAUNCH("k_rfft_axis");
+    }
 }
 
 // Grouped launches of planned stages: one launch per kMaxGrp argument sets, dynamic shared memory
@@ -1021,6 +1004,54 @@ static void launch_planned(const std::vector<Planned<A>>& ps, Kernel kernel, int
         kernel<<<total, threads, smem, st>>>(g);
         CNG_LAUNCH(what);
     });
+}
+
+// One transform stage of one problem; the stages of a group in one launch each.
+template <class R>
+struct ChebStage {
+    const c2<R>* in;
+    c2<R>* out;
+    long long ncols;
+    int N, M, maxseq;
+};
+template <class R>
+struct AxisStage {
+    const void* in;
+    void* out;
+    long long outer;
+    int inner, ncompact, L, maxseq;
+    Expand<R> ex;
+};
+
+template <class R>
+static void launch_cheb_group(const std::vector<ChebStage<R>>& js, bool forward, cudaStream_t st, int threads) {
+    if constexpr (sizeof(R) == 8) {
+        std::vector<FxChebJob> f;
+        for (const auto& j : js) f.push_back(FxChebJob{j.in, j.out, j.ncols, j.N, j.M, j.maxseq});
+        fx_cheb(f, forward, st, threads);
+    } else {
+        std::vector<Planned<ChebArgs<R>>> ps;
+        for (const auto& j : js) ps.push_back(plan_cheb<R>(j.in, j.out, j.ncols, j.N, j.M, forward, j.maxseq));
+        const auto kernel = forward ? k_cheb_fwd_grp<R> : k_cheb_bwd_grp<R>;
+        set_smem_attr<R>((const void*)kernel);
+        launch_planned(ps, kernel, threads > 0 ? threads : kFftThreads, st, "k_cheb_grp");
+    }
+}
+
+template <class R>
+static void launch_axis_group(const std::vector<AxisStage<R>>& js, bool real, bool forward, cudaStream_t st, int threads) {
+    if constexpr (sizeof(R) == 8) {
+        std::vector<FxAxisJob> f;
+        for (const auto& j : js) f.push_back(FxAxisJob{j.in, j.out, j.outer, j.inner, j.ncompact, j.L, j.maxseq, j.ex});
+        fx_axis(f, real, forward, st, threads);
+    } else {
+        std::vector<Planned<AxisArgs<R>>> ps;
+        for (const auto& j : js)
+            ps.push_back(plan_axis<R>(real, j.in, j.out, j.outer, j.inner, j.ncompact, j.L, forward, j.maxseq, j.ex));
+        const auto kernel = real ? k_rfft_axis_grp<R> : k_fft_axis_grp<R>;
+        set_smem_attr<R>((const void*)kernel);
+        launch_planned(ps, kernel, threads > 0 ? threads : kFftThreads, st, "k_axis_grp");
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1143,7 +1174,7 @@ void Rhs::run(const double2* state, double2* rows, cudaStream_t st) {
     C* A = static_cast<C*>(W1);
     C* Bf = static_cast<C*>(W2);
     const int ngy = dev.ngy * ncase, ngz = dev.ngz * ncase;
-    launch_cheb<R>(Sp, A, spec_cols(ngy), ny, my, false, st, maxseq, threads);
+    launch_cheb<R>(Sp, A, spec_cols(ngy), ny, my, false, st, maxseq, threads, ndir == 0);
     C* cur = A;
     C* other = Bf;
     // 3. z: the z-groups ((i kz)^oz of their y-group), then the z backward transform
@@ -1212,7 +1243,7 @@ void Rhs::run(const double2* state, double2* rows, cudaStream_t st) {
         std::swap(cur, other);
     }
     // 8. Chebyshev forward: [cols][my] -> S [cols][ny]
-    launch_cheb<R>(cur, Sp, spec_cols(no), ny, my, true, st, maxseq, threads);
+    launch_cheb<R>(cur, Sp, spec_cols(no), ny, my, true, st, maxseq, threads, ndir == 0);
     // 9. pack rows (every bucket in one launch) and add the constant part
     launch_pack<R>(&self, 1, rows, st);
     if (nb0) {
@@ -1228,12 +1259,12 @@ void Rhs::run(const double2* state, double2* rows, cudaStream_t st) {
 template <class R>
 void run_group(Rhs* const* hs, int n, const double2* state, double2* rows, cudaStream_t st) {
     using C = c2<R>;
-    const int threads = hs[0]->threads > 0 ? hs[0]->threads : kFftThreads;
+    const int threads = hs[0]->threads;
     const int ndir = hs[0]->ndir;
     for (int i = 0; i < n; ++i) {
         if (hs[i]->ndir != ndir || hs[i]->precision != hs[0]->precision)
             throw InvalidArgument("grouped F: every problem needs the same precision and Fourier directions");
-        if ((hs[i]->threads > 0 ? hs[i]->threads : kFftThreads) != threads)
+        if ((hs[i]->threads > 0 ? hs[i]->threads : kFftThreads) != (threads > 0 ? threads : kFftThreads))
             throw InvalidArgument("grouped F: every problem needs the same transform block size");
     }
     if (ndir < 1) throw InvalidArgument("grouped F: at least one Fourier direction");
@@ -1241,19 +1272,18 @@ void run_group(Rhs* const* hs, int n, const double2* state, double2* rows, cudaS
     launch_unpack<R>(hs, n, state, st);
     // the stages' buffers per problem, as Rhs::run rotates them
     std::vector<C*> cur(n), other(n);
-    std::vector<Planned<ChebArgs<R>>> cheb;
+    std::vector<ChebStage<R>> cheb;
     for (int i = 0; i < n; ++i) {
         const Rhs& h = *hs[i];
         cur[i] = static_cast<C*>(h.W1);
         other[i] = static_cast<C*>(h.W2);
         const long long cols = h.spec_cols(h.dev.ngy * h.ncase);
         if (h.ny == 1 && h.my == 1) throw InvalidArgument("grouped F: a Chebyshev direction is needed");
-        cheb.push_back(plan_cheb<R>(static_cast<const C*>(h.S), cur[i], cols, h.ny, h.my, false, h.maxseq));
+        cheb.push_back(ChebStage<R>{static_cast<const C*>(h.S), cur[i], cols, h.ny, h.my, h.maxseq});
     }
-    set_smem_attr<R>((const void*)k_cheb_bwd_grp<R>);
-    launch_planned(cheb, k_cheb_bwd_grp<R>, threads, st, "k_cheb_bwd_grp");
+    launch_cheb_group<R>(cheb, false, st, threads);
     if (ndir == 2) {
-        std::vector<Planned<AxisArgs<R>>> z;
+        std::vector<AxisStage<R>> z;
         for (int i = 0; i < n; ++i) {
             const Rhs& h = *hs[i];
             Expand<R> ez{};
@@ -1261,15 +1291,13 @@ void run_group(Rhs* const* hs, int n, const double2* state, double2* rows, cudaS
                 ez.nout = h.dev.ngz; ez.nin = h.dev.ngy; ez.per = h.Kx; ez.nidx = h.Nzc;
                 ez.src = h.dev.zg_y; ez.ord = h.dev.zg_oz; ez.tab = static_cast<const C*>(h.ktab_z);
             }
-            z.push_back(plan_axis<R>(false, cur[i], other[i], (long long)h.dev.ngz * h.ncase * h.Kx, h.my, h.Nzc,
-                                     h.mz, false, h.maxseq, ez));
+            z.push_back(AxisStage<R>{cur[i], other[i], (long long)h.dev.ngz * h.ncase * h.Kx, h.my, h.Nzc, h.mz, h.maxseq, ez});
             std::swap(cur[i], other[i]);
         }
-        set_smem_attr<R>((const void*)k_fft_axis_grp<R>);
-        launch_planned(z, k_fft_axis_grp<R>, threads, st, "k_fft_axis_grp");
+        launch_axis_group<R>(z, false, false, st, threads);
     }
     // x backward (c2r) with the x expansions
-    std::vector<Planned<AxisArgs<R>>> xb;
+    std::vector<AxisStage<R>> xb;
     std::vector<R*> G(n);
     for (int i = 0; i < n; ++i) {
         const Rhs& h = *hs[i];
@@ -1279,13 +1307,11 @@ void run_group(Rhs* const* hs, int n, const double2* state, double2* rows, cudaS
             exx.nout = h.nfactors; exx.nin = h.dev.ngz; exx.per = 1; exx.nidx = h.Kx;
             exx.src = h.dev.f_z; exx.ord = h.f_ox; exx.tab = static_cast<const C*>(h.ktab_x);
         }
-        xb.push_back(plan_axis<R>(true, cur[i], other[i], (long long)h.nfactors * h.ncase, (int)inner, h.Kx, h.mx,
-                                  false, h.maxseq, exx));
+        xb.push_back(AxisStage<R>{cur[i], other[i], (long long)h.nfactors * h.ncase, (int)inner, h.Kx, h.mx, h.maxseq, exx});
         G[i] = reinterpret_cast<R*>(other[i]);
         std::swap(cur[i], other[i]);
     }
-    set_smem_attr<R>((const void*)k_rfft_axis_grp<R>);
-    launch_planned(xb, k_rfft_axis_grp<R>, threads, st, "k_rfft_axis_grp(backward)");
+    launch_axis_group<R>(xb, true, false, st, threads);
     // products
     {
         constexpr int VV = sizeof(R) == 4 ? 4 : 2;
@@ -1308,34 +1334,30 @@ void run_group(Rhs* const* hs, int n, const double2* state, double2* rows, cudaS
         });
     }
     // x forward (r2c)
-    std::vector<Planned<AxisArgs<R>>> xf;
+    std::vector<AxisStage<R>> xf;
     for (int i = 0; i < n; ++i) {
         const Rhs& h = *hs[i];
         const long long inner = (long long)(ndir == 2 ? h.mz : 1) * h.my;
-        xf.push_back(plan_axis<R>(true, cur[i], other[i], (long long)h.noutputs * h.ncase, (int)inner, h.Kx, h.mx,
-                                  true, h.maxseq, Expand<R>{}));
+        xf.push_back(AxisStage<R>{cur[i], other[i], (long long)h.noutputs * h.ncase, (int)inner, h.Kx, h.mx, h.maxseq, {}});
         std::swap(cur[i], other[i]);
     }
-    launch_planned(xf, k_rfft_axis_grp<R>, threads, st, "k_rfft_axis_grp(forward)");
+    launch_axis_group<R>(xf, true, true, st, threads);
     if (ndir == 2) {
-        std::vector<Planned<AxisArgs<R>>> z;
+        std::vector<AxisStage<R>> z;
         for (int i = 0; i < n; ++i) {
             const Rhs& h = *hs[i];
-            z.push_back(plan_axis<R>(false, cur[i], other[i], (long long)h.noutputs * h.ncase * h.Kx, h.my, h.Nzc,
-                                     h.mz, true, h.maxseq, Expand<R>{}));
+            z.push_back(AxisStage<R>{cur[i], other[i], (long long)h.noutputs * h.ncase * h.Kx, h.my, h.Nzc, h.mz, h.maxseq, {}});
             std::swap(cur[i], other[i]);
         }
-        launch_planned(z, k_fft_axis_grp<R>, threads, st, "k_fft_axis_grp(forward)");
+        launch_axis_group<R>(z, false, true, st, threads);
     }
     // Chebyshev forward into S
     cheb.clear();
     for (int i = 0; i < n; ++i) {
         const Rhs& h = *hs[i];
-        cheb.push_back(plan_cheb<R>(cur[i], static_cast<C*>(h.S), h.spec_cols(h.noutputs * h.ncase), h.ny, h.my,
-                                    true, h.maxseq));
+        cheb.push_back(ChebStage<R>{cur[i], static_cast<C*>(h.S), h.spec_cols(h.noutputs * h.ncase), h.ny, h.my, h.maxseq});
     }
-    set_smem_attr<R>((const void*)k_cheb_fwd_grp<R>);
-    launch_planned(cheb, k_cheb_fwd_grp<R>, threads, st, "k_cheb_fwd_grp");
+    launch_cheb_group<R>(cheb, true, st, threads);
     // pack and the constant parts
     {
         launch_pack<R>(hs, n, rows, st);
