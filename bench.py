@@ -176,6 +176,8 @@ def solve_kernel(sched: int) -> str:
         return "k_solve_window_multi"
     if sched in autotune.partitioned_schedules():
         return "k_solve_part"
+    if sched in autotune.scheduled_schedules():
+        return "k_solve_flow"
     if sched in autotune.split_schedules():
         return "k_solve_split_multi"
     return "k_solve_compact_multi"

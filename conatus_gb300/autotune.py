@@ -4,10 +4,9 @@ Candidates: the band kernel (one warp per system over the LU band, ``cng_banded_
 -1)``) and the compact-stream schedules of ``cng_banded_schedules`` (two systems per warp over the
 union pattern of the factors, with different staging chunks and ring depths, over whole vectors
 or over windows of them with the rest in a scratch (more resident warps, the same bits); one
-system per warp with the lanes split over entries and components for small batches; and the
-partitioned solve of small FP64 batches, one block of warps per system sweeping its blocks of 32
-columns at once). The
-partitioned solve is a candidate only where the DeviceProblem opts into it (``dev.partitioned``,
+system per warp with the lanes split over entries and components for small batches; the same operations
+by time slots fixed at the factorization, a warp per system; and the partitioned solve of small FP64 batches, one
+block of warps per system sweeping its blocks of 32 columns at once). The partitioned solve is a candidate only where the DeviceProblem opts into it (``dev.partitioned``,
 or CONATUS_GB300_PARTITIONED=1): its residuals run up to about 15x those of the sequential sweeps.
 Candidates a factor set cannot take (a shared pair, the FP32 form, a batch too large for the
 partitioned solve's responses) are refused by the library and skipped. Each candidate solves
@@ -26,11 +25,12 @@ The reference chooses its solve kernel by constructor flags (python/conatus/runt
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 from ._lib import call
 
-__all__ = ["schedules", "split_schedules", "partitioned_schedules", "windowed_schedules", "tune_solve", "tune_rhs",
+__all__ = ["schedules", "split_schedules", "scheduled_schedules", "partitioned_schedules", "windowed_schedules", "tune_solve", "tune_rhs",
            "cache"]
 
 _CACHE: dict = {}
@@ -57,6 +57,14 @@ def split_schedules() -> set:
     latency variant: the same sweeps, another order of sums in the border correction), and the
     partitioned solve."""
     return {k for k, f in enumerate(_flags()) if f in (1, 2)}
+
+
+@functools.lru_cache(maxsize=None)
+def scheduled_schedules() -> tuple:
+    """The scheduled solve: (with the split-lane schedules' results bit for bit and like them no shared
+    pairs; with schedule 0's, shared pairs as well)."""
+    n = len(_flags())
+    return n - 2, n - 1
 
 
 def partitioned_schedules() -> set:
@@ -109,6 +117,10 @@ def tune_solve(dev, key, fs, stream=None, reps: int = 3, candidates=None) -> dic
         if not getattr(dev, "partitioned", False):       # opted into (its residuals run larger)
             part = partitioned_schedules()
             candidates = [c for c in candidates if c not in part]
+        if getattr(dev, "d", 1) == 0:
+            # one system, whose tau matrix hands each rounding on some 1e5 times larger: the border sums
+            # keep one order (the two scheduled solves take the same time)
+            candidates = [c for c in candidates if c != scheduled_schedules()[1]]
     if stream is None:
         st = torch.cuda.current_stream()
     elif isinstance(stream, int):

@@ -244,8 +244,8 @@ class _BandedBatch:
     capacitance_cond_max = property(lambda self: self._h.cond_max)
     col_border = property(lambda self: False)
     col_border_nnz = property(lambda self: 0)
-    # the GB300 solve reads the band directly (one warp per system); no level schedule is built,
-    # so the reference's level-schedule diagnostics (module.cpp:356-373) report none
+    # the reference's level schedules are not built (the scheduled solve's time slots are of single
+    # operations), so its level-schedule diagnostics (module.cpp:356-373) report none
     level_scheduled = property(lambda self: False)
     level_transposed = property(lambda self: False)
     level_merged = property(lambda self: False)

@@ -28,10 +28,15 @@
 
 #include "common.cuh"
 #include "conatus_gb300.h"
+#include "flow_solve.cuh"
+#include "real_form.cuh"
+#include "small_lu.cuh"
+#include "solve_io.cuh"
 
 namespace cng {
 
 static constexpr int kWarpsPerBlock = 4;
+static constexpr size_t kFlowAutoBytes = (size_t)1 << 30;     // most bytes of operations a host-built handle adds
 static constexpr size_t kMaxSolveSmem = 200 * 1024;   // bytes of shared memory for the y vectors
 
 template <class T>
@@ -235,25 +240,6 @@ __device__ int small_getrf(T* a, int* piv, int r) {
     if (info == 0)
         for (int k = 0; k < r; ++k) a[k * r + k] = one<T>() / a[k * r + k];
     return info;
-}
-
-// z := S^{-1} z with the small LU (getrs 'N'), lane 0.
-template <class T>
-__device__ void small_getrs(const T* a, const int* piv, T* z, int r) {
-    for (int k = 0; k < r; ++k) {
-        const int p = piv[k];
-        if (p != k) {
-            T t = z[k];
-            z[k] = z[p];
-            z[p] = t;
-        }
-    }
-    for (int k = 0; k < r; ++k)
-        for (int i = k + 1; i < r; ++i) z[i] = z[i] - a[k * r + i] * z[k];
-    for (int k = r - 1; k >= 0; --k) {
-        z[k] = z[k] * a[k * r + k];
-        for (int i = 0; i < k; ++i) z[i] = z[i] - a[k * r + i] * z[k];
-    }
 }
 
 // z := S^{-1} z with the small LU staged in shared memory (lane 0; r <= kMaxRUnroll): the
@@ -539,50 +525,6 @@ __device__ void warp_band_solve_staged(const T* __restrict__ ab, const int* __re
     }
 }
 
-// Input/output adapters of the solve kernel: plain in-place, mapped (int64 gather/scatter maps)
-// and split (complex system with real data: b = re[rows_c] + i re[rows_s]).
-enum IoKind { IO_PLAIN = 0, IO_MAPPED = 1, IO_SPLIT = 2, IO_MIXED = 3 };
-
-struct SolveIo {
-    const void* rhs;
-    void* x;
-    const long long* rows;
-    const long long* cols;
-    const long long* rows_s;
-    const long long* cols_s;
-    int accumulate = 0;
-    void* xT = nullptr;            // IO_MIXED: x also written row-major over the systems, [n][batch]
-};
-
-template <class T, int IO>
-__device__ inline T io_load(const SolveIo& io, int sys, int n, int i) {
-    const size_t k = (size_t)sys * n + i;
-    if constexpr (IO == IO_PLAIN) {
-        return static_cast<const T*>(io.rhs)[k];
-    } else if constexpr (IO == IO_MAPPED) {
-        const T* rhs = static_cast<const T*>(io.rhs);
-        return rhs[io.rows ? io.rows[k] : (long long)k];
-    } else {
-        const double* re = static_cast<const double*>(io.rhs);
-        return T(zd(re[io.rows[k]], re[io.rows_s[k]]));
-    }
-}
-
-template <class T, int IO>
-__device__ inline void io_store(const SolveIo& io, int sys, int n, int i, T v) {
-    const size_t k = (size_t)sys * n + i;
-    if constexpr (IO == IO_PLAIN) {
-        static_cast<T*>(io.x)[k] = v;
-    } else if constexpr (IO == IO_MAPPED) {
-        static_cast<T*>(io.x)[io.cols ? io.cols[k] : (long long)k] = v;
-    } else {
-        double* x = static_cast<double*>(io.x);
-        const zd z = *reinterpret_cast<const zd*>(&v);
-        x[io.cols[k]] = z.re;
-        x[io.cols_s[k]] = z.im;
-    }
-}
-
 template <class T, int IO>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_solve(BandView<T> v, SolveIo io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -782,6 +724,12 @@ struct Banded {
     zf* w32 = nullptr;
     zf* slu32 = nullptr;
     bool fp32_ready = false;
+    // complex handles whose systems are real up to powers of i (real_form.cuh): phases of the rows (in
+    // solver order) and columns, and the scheduled solve built on them (kFlow32, kFlow16)
+    bool real_form = false;
+    unsigned char* rowp = nullptr;
+    unsigned char* colp = nullptr;
+    std::unique_ptr<FlowForm> flow;
     // shared-pattern refactorization data (create_shared)
     int nnz = 0;
     long long* bulk_dest = nullptr;
@@ -795,7 +743,8 @@ struct Banded {
                         (void*)bp, (void*)bcol, (void*)ab32, (void*)vt32, (void*)w32, (void*)slu32,
                         (void*)c_offL, (void*)c_Lrow, (void*)c_Lmask, (void*)c_offU, (void*)c_Udist,
                         (void*)c_offV, (void*)c_Vcol, c_L, c_U, c_V, (void*)c_piv, (void*)c_L32,
-                        (void*)c_U32, (void*)c_V32, (void*)flip_r, (void*)flip_c, p_Rf, p_Rb, w_scr})
+                        (void*)c_U32, (void*)c_V32, (void*)flip_r, (void*)flip_c, p_Rf, p_Rb, w_scr, (void*)rowp,
+                        (void*)colp})
             dev_free(p);
     }
 
@@ -899,6 +848,35 @@ static void finish_factor(Banded& h, cudaStream_t st, cudaEvent_t e0, cudaEvent_
             throw RuntimeFailure("BandedBatch: capacitance condition number is NaN");
         if (!(cond[k] <= h.cond_max)) h.cond_max = cond[k];
     }
+}
+
+// the phases of the real form, from the assembled systems (before launch_factor)
+static void detect_phases(Banded& h, cudaStream_t st) {
+    h.real_form = false;
+    if (h.dtype != 1) return;
+    std::vector<unsigned char> row, col;
+    if (!find_phases(static_cast<const zd*>(h.ab), static_cast<const zd*>(h.vt), h.batch, h.n, h.r, h.kl + h.ku, h.ldab,
+                     st, row, col))
+        return;
+    if (!h.rowp) {
+        dalloc(&h.rowp, h.n, 1);
+        dalloc(&h.colp, h.n, 1);
+    }
+    CNG_CUDA(cudaMemcpyAsync(h.rowp, row.data(), h.n, cudaMemcpyHostToDevice, st));
+    CNG_CUDA(cudaMemcpyAsync(h.colp, col.data(), h.n, cudaMemcpyHostToDevice, st));
+    CNG_CUDA(cudaStreamSynchronize(st));
+    h.real_form = true;
+}
+
+// the scheduled solve of the factors at hand (refused with InvalidArgument where it does not apply)
+static void build_flow(Banded& h, int lanes, cudaStream_t st) {
+    bool in_order = true;
+    for (int i = 0; i < h.n; ++i) in_order = in_order && h.perm_host[i] == i;
+    const FlowSource s{h.dtype, h.batch, h.n, h.r, h.kl, h.ku, h.ldab, h.ab, h.ipiv, h.vt, h.w, h.slu, h.spiv, h.perm, in_order,
+                       h.real_form ? h.rowp : nullptr, h.real_form ? h.colp : nullptr,
+                       h.shared ? h.flip_r : nullptr, h.shared ? h.flip_c : nullptr, h.fp32_ready, lanes};
+    h.flow.reset();
+    h.flow = flow_build(s, st);
 }
 
 static void launch_factor(Banded& h, cudaStream_t st) {
@@ -1079,6 +1057,10 @@ static void launch_solve_t(const Banded& h, const SolveIo& io, cudaStream_t st) 
 static bool launch_solve_compact(const Banded& h, int io_kind, const SolveIo& io, cudaStream_t st);
 
 static void launch_solve(const Banded& h, int io_kind, const SolveIo& io, cudaStream_t st) {
+    if (h.flow) {
+        flow_solve({FlowJob{h.flow.get(), io, SolveIo{}, 0, h.batch}}, io_kind, st);
+        return;
+    }
     if (h.compact_ready && h.sched >= 0 && launch_solve_compact(h, io_kind, io, st)) return;
     if (h.dtype == 0) {
         if (io_kind == IO_PLAIN) launch_solve_t<double, IO_PLAIN>(h, io, st);
@@ -1123,6 +1105,7 @@ static void make_fp32(Banded& h, cudaStream_t st) {
     if (h.compact_ready) demote_compact(h, st);
     CNG_CUDA(cudaStreamSynchronize(st));
     h.fp32_ready = true;
+    if (h.flow) build_flow(h, h.flow->lanes, st);
 }
 
 static void prepare_transpose(Banded& h, cudaStream_t st) {
@@ -1228,10 +1211,19 @@ int cng_banded_create_csr(int dtype, int batch, int n, const int32_t* indptr, co
             build_csr<zd>(*h, indptr, indices, static_cast<const zd*>(data),
                           reinterpret_cast<const long long*>(nnz_offsets), border, st);
         check_smem(*h);
+        detect_phases(*h, st);
         EventPair ev;
         CNG_CUDA(cudaEventRecord(ev.e0, st));
         launch_factor(*h, st);
         finish_factor(*h, st, ev.e0, ev.e1);
+        // n = 262 complex, 128 systems: the band kernel takes 570 us. What the form does not take (values
+        // that are not real up to powers of i) and what it would need too much memory for stay with it
+        if ((size_t)h->batch * n * kFlowColumnBytes <= kFlowAutoBytes) {
+            try {
+                build_flow(*h, 32, st);
+            } catch (const InvalidArgument&) {
+            }
+        }
         *out = reinterpret_cast<cng_banded*>(h.release());
     })
 }
@@ -1256,6 +1248,7 @@ int cng_banded_create_shared(int dtype, int batch, int n, const int32_t* indptr,
         EventPair ev;
         CNG_CUDA(cudaEventRecord(ev.e0, st));
         launch_layout_shared(*h, values, st);
+        detect_phases(*h, st);
         launch_factor(*h, st);
         finish_factor(*h, st, ev.e0, ev.e1);
         *out = reinterpret_cast<cng_banded*>(h.release());
@@ -1412,6 +1405,11 @@ int cng_banded_solve_fp32(const cng_banded* hh, const void* b, void* x, int accu
         if (!h->fp32_ready) throw InvalidArgument("call cng_banded_make_fp32 first (it allocates)");
         if (!b || !x) throw InvalidArgument("null device pointer");
         if (b == x) throw InvalidArgument("b and x must not alias");
+        if (h->flow && h->flow->data[1]) {
+            SolveIo io{b, x, nullptr, nullptr, nullptr, nullptr, accumulate};
+            flow_solve({FlowJob{h->flow.get(), io, SolveIo{}, 0, h->batch}}, IO_MIXED, static_cast<cudaStream_t>(stream));
+            return CNG_OK;
+        }
         if (h->compact_ready && h->sched >= 0) {
             SolveIo io{b, x, nullptr, nullptr, nullptr, nullptr, accumulate};
             launch_solve_compact(*h, IO_MIXED, io, static_cast<cudaStream_t>(stream));
@@ -1430,9 +1428,18 @@ int cng_banded_refactor_shared(cng_banded* hh, const void* values, void* stream)
         EventPair ev;
         CNG_CUDA(cudaEventRecord(ev.e0, st));
         launch_layout_shared(*h, values, st);
+        detect_phases(*h, st);
         launch_factor(*h, st);
         h->transposed_ready = false;
         finish_factor(*h, st, ev.e0, ev.e1);
+        if (h->flow) {
+            try {
+                build_flow(*h, h->flow->lanes, st);
+            } catch (const InvalidArgument&) {   // the new values do not take the form: the band kernel
+                h->flow.reset();
+                h->sched = -1;
+            }
+        }
         if (h->fp32_ready) make_fp32(*h, st);
     })
 }
@@ -1473,14 +1480,18 @@ constexpr int kCChunk = 8;              // columns per staged chunk (the default
 // resident warps per SM; the same bits as schedule 0); 16-18 the same with 8 lanes per system
 // (four systems, two warp groups of the streams per warp: fewer instructions per system).
 struct CompactSchedule { int chunk, stages, split, lanes = 16; };
-constexpr int kNumSchedules = 19;
+// Schedules 19 and 20 are the scheduled solve (flow_solve.cu, the sweeps' operations by time slots on the
+// real form, a warp per system): 19 (split = 1) with the split-lane schedules' results, bit for bit, and
+// like them no shared pairs; 20 with schedule 0's, shared pairs as well.
+constexpr int kNumSchedules = 21;
 constexpr int kPartSchedule = 11;
+constexpr int kFlow32 = 19, kFlow16 = 20;
 constexpr int kWindowFlag = 3;
 constexpr CompactSchedule kSchedules[kNumSchedules] = {{8, 2, 0}, {8, 3, 0}, {4, 3, 0}, {16, 2, 0},
                                                        {16, 3, 0}, {4, 4, 0}, {2, 4, 0}, {16, 4, 0},
                                                        {8, 2, 1}, {16, 2, 1}, {4, 3, 1}, {8, 2, 2},
                                                        {8, 2, 3}, {4, 3, 3}, {16, 2, 3}, {8, 3, 3},
-                                                       {8, 2, 3, 8}, {4, 3, 3, 8}, {8, 3, 3, 8}};
+                                                       {8, 2, 3, 8}, {4, 3, 3, 8}, {8, 3, 3, 8}, {16, 3, 1}, {16, 3, 0}};
 constexpr int kChunkSizes[4] = {2, 4, 8, 16};
 __host__ __device__ constexpr int chunk_index(int ch) { return ch == 2 ? 0 : (ch == 4 ? 1 : (ch == 8 ? 2 : 3)); }
 
@@ -3252,6 +3263,17 @@ static void launch_multi(const std::vector<const Banded*>& hs, const std::vector
             if constexpr (std::is_same<TF, zd>::value) launch_part(hs, ios, ios2, rng, st);
             else throw InvalidArgument("the partitioned solve is FP64 only: another schedule for the FP32 form");
             break;
+        case kFlow32:
+        case kFlow16: {
+            std::vector<FlowJob> jobs;
+            for (size_t i = 0; i < hs.size(); ++i) {
+                if (!hs[i]->flow) throw InvalidArgument("the scheduled solve is not built (cng_banded_set_schedule)");
+                const bool all = rng[2 * i + 1] < 0;
+                jobs.push_back(FlowJob{hs[i]->flow.get(), ios[i], ios2[i], all ? 0 : rng[2 * i], all ? hs[i]->batch : rng[2 * i + 1]});
+            }
+            flow_solve(jobs, IO, st);
+            break;
+        }
         case 12: launch_multi_t<TF, TD, IO, 8, 2, true>(hs, cds, ios, ios2, rng, sched, st); break;
         case 13: launch_multi_t<TF, TD, IO, 4, 3, true>(hs, cds, ios, ios2, rng, sched, st); break;
         case 14: launch_multi_t<TF, TD, IO, 16, 2, true>(hs, cds, ios, ios2, rng, sched, st); break;
@@ -3408,6 +3430,14 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
         if (!h) throw InvalidArgument("null handle");
         if (sched < -1 || sched >= kNumSchedules) throw InvalidArgument("schedule out of range");
         if (sched >= 0 && !h->compact_ready) throw InvalidArgument("compact schedules need cng_banded_compact first");
+        if (sched == cng::kFlow32 || sched == cng::kFlow16) {
+            const int lanes = sched == cng::kFlow32 ? 32 : 16;       // of a border sum
+            if (lanes == 32 && h->shared)
+                throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
+            if (!h->flow || h->flow->lanes != lanes) cng::build_flow(*h, lanes, nullptr);
+        } else {
+            h->flow.reset();                       // another schedule: the operations are not kept
+        }
         if (sched == cng::kPartSchedule) {
             cng::build_part(*h);                   // the responses (refused where it does not apply)
         } else if (h->part_ready) {                // another schedule: the responses are not kept

@@ -1,0 +1,61 @@
+// The scheduled solve (flow_solve.cu): built from a factorization, launched for several buckets at once.
+#pragma once
+
+#include <memory>
+#include <vector>
+
+#include "common.cuh"
+#include "solve_io.cuh"
+
+namespace cng {
+
+// the most bytes of operations of a system per column; more are refused (memory.py plans them)
+constexpr int kFlowColumnBytes = 400;
+
+struct FlowSource {                      // the factored handle's arrays (banded.cu)
+    int dtype, batch, n, r, kl, ku, ldab;
+    const void* ab;
+    const int* ipiv;
+    const void* vt;
+    const void* w;
+    const void* slu;
+    const int* spiv;
+    const int* perm;
+    bool in_order;                       // perm is the identity
+    const unsigned char* rowp;           // phases of the real form (complex handles)
+    const unsigned char* colp;
+    const unsigned char* flip_r;         // a shared pair's signs (NULL: no partner)
+    const unsigned char* flip_c;
+    bool fp32;                           // also the FP32 copies (mixed form)
+    int lanes;                           // lanes of a border sum: 16 or 32
+};
+
+struct FlowForm {
+    int n = 0, batch = 0, dtype = 0, lanes = 0;
+    int rows = 0;                        // rows of a system's vector: n, the border's sums, a zero
+    int ncr = 0;                         // right-hand sides of a factor: components x (system, partner)
+    int chunks = 0;                      // largest number of chunks of operations of a system
+    size_t sb[2] = {0, 0};               // bytes of a system: FP64, FP32
+    unsigned char* data[2] = {nullptr, nullptr};
+    int* nchunk = nullptr;               // per system
+    unsigned short* row = nullptr;       // [batch][n]: the row of each column
+    const int* perm = nullptr;           // NULL: the rows as they come
+    unsigned char* flags = nullptr;      // [2][n]: rows' and columns' phase | partner's sign << 1
+    ~FlowForm();
+    FlowForm() = default;
+    FlowForm(const FlowForm&) = delete;
+    FlowForm& operator=(const FlowForm&) = delete;
+};
+
+// Throws InvalidArgument where the form does not apply (size, fill, or values that are not real up to
+// the phases). Waits for `st`.
+std::unique_ptr<FlowForm> flow_build(const FlowSource& s, cudaStream_t st);
+
+struct FlowJob {
+    const FlowForm* form;
+    SolveIo io, io2;                     // io2: the partner (rhs NULL: none)
+    int s0, s1;                          // systems solved
+};
+void flow_solve(const std::vector<FlowJob>& jobs, int io_kind, cudaStream_t st);
+
+}  // namespace cng

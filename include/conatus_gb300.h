@@ -149,7 +149,7 @@ int cng_banded_solve_batch2(int nh, cng_banded* const* h, const void* const* b, 
 /* Schedules of the compact solve (the batched-solve kernel of the step): count, and per schedule
  * the columns per staged chunk of the factor streams, the depth of the staging ring and whether it
  * runs one system per warp with the lanes split over entries and real/imaginary parts (split = 1:
- * the latency variant for small batches; split = 2: the partitioned solve of small FP64 batches,
+ * the latency variants for small batches, the last of them by time slots as below; split = 2: the partitioned solve of small FP64 batches,
  * one block of warps per system sweeping its blocks of 32 columns at once; split = 3: the windowed
  * sweeps of two or four systems per warp, a window of each vector in shared memory and the rest in
  * a scratch, the same bits as schedule 0; else two systems per warp). Any output may be NULL. No
@@ -160,6 +160,13 @@ int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_
 /* Schedule of a handle: 0 .. count-1 a compact schedule (needs cng_banded_compact), -1 the band
  * kernel (one warp per system, no compact streams). cng_banded_solve_batch uses the handles'
  * common schedule (schedule 0 when they differ; the band kernel per bucket when all are -1).
+ * The last two schedules run the sweeps' operations by time slots fixed at the factorization, a warp
+ * per system: the last but one (split = 1) with the results of the split-lane schedules, bit for bit,
+ * the last with those of schedule 0, shared pairs and FP32 factors as well. Setting one builds its
+ * operations (allocates, runs on the legacy default stream and waits for it; freed when another
+ * schedule is set) and refuses (status 1) systems that are not real up to powers of i and more than
+ * 400 bytes of operations per column. Handles of cng_banded_create_csr hold them from the start where
+ * they apply (up to 1 GB), in place of the band kernel's solve.
  * Setting the partitioned schedule builds its responses to unit window values (allocates, runs on
  * the legacy default stream and waits for it) and refuses (status 1) shared pairs, kl > 16,
  * kl + ku > 32, n > 1024 and responses above 256 MB; its solves refuse the FP32 factors and
