@@ -8,7 +8,8 @@
 // scheduling: Graham 1966; sparse triangular solves by levels: Anderson and Saad 1989), `flow_ops` of
 // them to a slot, and a warp runs slot after slot, a lane per (operation, component). An operation is
 // a fused multiply-add v_dst = -c v_src + v_dst (or + 0). The rows of the vector v stay where they are:
-// the interchanges only decide which rows an operation names. The border's sums, the small LU solve
+// the interchanges only decide which rows an operation names (a row is named by the column it ends up
+// the pivot row of, so the solution comes out in order). The border's sums, the small LU solve
 // and the correction x - W z are operations as well (the rows behind the system's hold the partial
 // sums). L and U take about n / 2 slots each: the two parities of the Chebyshev modes are independent,
 // and so are most rows of a column.
@@ -37,7 +38,7 @@ constexpr int kMaxBorder = 64;
 constexpr unsigned kFresh = 0x80000000u;         // the operation's sum starts from 0
 
 __host__ __device__ constexpr int flow_ops(int ncr) { return 32 / ncr; }        // operations of a slot
-// a chunk: values [kSlots][ops], then rows [kSlots][ops] (read | written << 16 | kFresh)
+// a chunk: values -c [kSlots][ops], then rows [kSlots][ops] (read | written << 16 | kFresh)
 __host__ __device__ constexpr int flow_chunk(int ncr, int elem) { return kSlots * flow_ops(ncr) * (elem + 4); }
 
 FlowForm::~FlowForm() {
@@ -104,7 +105,7 @@ struct FlowPlan {
                 if constexpr (!COUNT) {
                     unsigned char* ch = data + (size_t)(t / kSlots) * chunk;
                     const int e = (t % kSlots) * ops + at + rank;
-                    reinterpret_cast<R*>(ch)[e] = (R)c;
+                    reinterpret_cast<R*>(ch)[e] = (R)(-c);
                     reinterpret_cast<unsigned*>(ch + (size_t)kSlots * ops * sizeof(R))[e] =
                         (unsigned)src | (unsigned)dst << 16 | (fresh ? kFresh : 0u);
                 }
@@ -134,7 +135,8 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
     put.read = put.ready + rows;
     unsigned short* ord = reinterpret_cast<unsigned short*>(put.read + rows);      // row at a position
     unsigned short* piv = ord + n;
-    put.next = piv + n;
+    unsigned short* name = piv + n;
+    put.next = name + n;
     put.cnt = reinterpret_cast<unsigned char*>(put.next + in.cap + 1);
     unsigned char* rowph = put.cnt + in.cap;
     put.data = COUNT ? nullptr : o.data + (size_t)sys * o.sb;
@@ -155,6 +157,21 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
     for (int j = lane; j < n; j += 32) {
         piv[j] = (unsigned short)ipiv[j];
         rowph[j] = (unsigned char)(phase_of(q, j) ^ (pure_imag(ab[(size_t)j * ldab + kv]) ? 1 : 0));
+    }
+    __syncwarp();
+    if (lane == 0) {                             // where every row ends up
+        for (int j = 0; j + 1 < n; ++j) {
+            const int l = piv[j];
+            const unsigned short t = ord[j];
+            ord[j] = ord[l];
+            ord[l] = t;
+        }
+        for (int j = 0; j < n; ++j) name[ord[j]] = (unsigned short)j;
+    }
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        ord[i] = name[i];                        // from here on the name of the row at a position
+        if constexpr (!COUNT) o.row[(size_t)sys * n + i] = name[i];
     }
     __syncwarp();
     auto dinv_of = [&](int j) { return real_part_of(ab[(size_t)j * ldab + kv], phase_of(q, j) - rowph[j], bad); };
@@ -196,9 +213,8 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
         }
     }
     for (int j0 = 0; j0 < n; j0 += 32) {         // x_j = y_j / u_jj, in y_j's row
-        const int j = j0 + lane, at = j < n ? ord[j] : 0;
+        const int j = j0 + lane, at = j < n ? j : 0;
         put(j < n, at, at, j < n ? -dinv_of(j) : 0.0, true);
-        if (!COUNT && j < n) o.row[(size_t)sys * n + j] = (unsigned short)at;
     }
     // the border: rows n + a LS + l hold the partial sums of border row a, row n + r LS + i a product
     const T* vt = in.vt + (size_t)sys * r * n;
@@ -215,7 +231,7 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
             for (int h = 0; h < 32; h += LS) {
                 const bool mine = v != 0.0 && e - e0 >= h && e - e0 < h + LS;
                 const bool fresh = mine && put.ready[sum + l] == 0;
-                put(mine, mine ? ord[j] : 0, mine ? sum + l : 0, -v, fresh);
+                put(mine, mine ? j : 0, mine ? sum + l : 0, -v, fresh);
             }
             e0 += __popc(m);
         }
@@ -268,7 +284,7 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
             for (int j0 = 0; j0 < n; j0 += 32) {
                 const int j = j0 + lane;
                 const double v = j < n ? real_part_of(w[(size_t)k * n + j], phase_of(q, j) - phase_of(p, k), bad) : 0.0;
-                put(v != 0.0, z(k), v != 0.0 ? ord[j] : 0, v, false);
+                put(v != 0.0, z(k), v != 0.0 ? j : 0, v, false);
             }
     }
     if constexpr (COUNT) {
@@ -323,7 +339,7 @@ static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
         throw InvalidArgument("scheduled solve: system too large for shared memory");
     const int ops = flow_ops(f->ncr);
     const int cap = std::min(65000, kFlowColumnBytes * (n + 64) / (12 * ops) / kSlots * kSlots);
-    const size_t smem = (size_t)f->rows * 8 + (size_t)n * 5 + (size_t)cap * 3 + 2;
+    const size_t smem = (size_t)f->rows * 8 + (size_t)n * 7 + (size_t)cap * 3 + 2;
     if (smem > kFlowSmem) throw InvalidArgument("scheduled solve: system too large");
     ensure_smem_attr((const void*)k_flow_build<T, double, true>, (int)kFlowSmem);
     ensure_smem_attr((const void*)k_flow_build<T, double, false>, (int)kFlowSmem);
@@ -391,7 +407,7 @@ std::unique_ptr<FlowForm> flow_build(const FlowSource& s, cudaStream_t st) {
 
 // ---- solve ---------------------------------------------------------------------------------------
 struct FlowArgs {
-    int n, rows, batch, s0, s1;
+    int n, rows, ncr, batch, s0, s1;
     size_t sb;
     const unsigned char* data;
     const int *nchunk, *perm;
@@ -409,17 +425,14 @@ __device__ __forceinline__ float flow_fma(float a, float b, float c) { return fm
 
 // A warp per system or shared pair. NCR: right-hand sides of a factor (1: real, 2: complex, 4: a pair)
 template <class R, int NCR, int IO>
-__global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_constant__ FlowMulti ms, int smem_sys) {
+__device__ __forceinline__ void flow_body(const FlowArgs& a, int block, int smem_sys) {
     extern __shared__ __align__(16) unsigned char fsm[];
     constexpr int NC = NCR == 1 ? 1 : 2;         // components of an entry
     constexpr int OPS = flow_ops(NCR), CHB = flow_chunk(NCR, (int)sizeof(R));
     static_assert(CHB % 512 == 0, "a warp copies whole rows of a chunk");
     using V = std::conditional_t<NC == 1, double, std::conditional_t<sizeof(R) == 8, zd, zf>>;
-    int bk = 0;
-    while (bk + 1 < ms.nb && (int)blockIdx.x >= ms.start[bk + 1]) ++bk;
-    const FlowArgs& a = ms.a[bk];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int sys = a.s0 + ((int)blockIdx.x - ms.start[bk]) * ((int)blockDim.x / 32) + wib;
+    const int sys = a.s0 + block * ((int)blockDim.x / 32) + wib;
     if (sys >= a.s1) return;                     // the whole warp
     const int n = a.n;
     unsigned char* ring = fsm + (size_t)wib * smem_sys;
@@ -439,13 +452,15 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_con
     for (int c = 0; c < kRing - 1; ++c) stage(c);
     // the right-hand sides, rows in solver order, times i^-p and the partner's signs
     constexpr int kU = 8;                        // rows in flight a lane
+    const unsigned short* row = a.row + (size_t)sys * n;
     for (int i0 = lane; i0 < n; i0 += kU * 32) {
-        int p[kU];
+        int p[kU], at[kU];
         unsigned char fl[kU];
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int i = min(i0 + u * 32, n - 1);
+            const int i = min(i0 + u * 32, n - 1);                // the last row again: the same value
             p[u] = a.perm ? a.perm[i] : i;
+            at[u] = row[i];
             fl[u] = a.in[i];
         }
         V v[kU], v2[kU];
@@ -462,12 +477,11 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_con
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int i = min(i0 + u * 32, n - 1);                // the last row again: the same value
             if constexpr (NC == 1) {
-                y[i] = v[u];
+                y[at[u]] = v[u];
             } else {
-                reinterpret_cast<V*>(y)[i * (NCR / 2)] = phase_in(v[u], fl[u] & 1);
-                if constexpr (NCR == 4) reinterpret_cast<V*>(y)[i * 2 + 1] = phase_in(fl[u] & 2 ? -v2[u] : v2[u], fl[u] & 1);
+                reinterpret_cast<V*>(y)[at[u] * (NCR / 2)] = phase_in(v[u], fl[u] & 1);
+                if constexpr (NCR == 4) reinterpret_cast<V*>(y)[at[u] * 2 + 1] = phase_in(fl[u] & 2 ? -v2[u] : v2[u], fl[u] & 1);
             }
         }
     }
@@ -492,7 +506,7 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_con
                 src = yc + (w & 0xffffu) * NCR;
                 dst = yc + ((w >> 16) & 0x7fffu) * NCR;
                 add = w & kFresh ? zero : dst;
-                v = -x;
+                v = x;
             };
             unsigned w = rows[OPS];
             R x = val[OPS];
@@ -512,25 +526,19 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_con
         }
     }
     // the solution, times i^q and the partner's signs, a lane per component
-    const unsigned short* row = a.row + (size_t)sys * n;
     const int comp = lane % NCR, im = comp & 1;
     const bool partner = comp >= 2;
     const SolveIo io = partner ? a.io2 : a.io;
     const size_t k0 = (size_t)sys * n;
     double* xs = static_cast<double*>(io.x) + (IO == IO_SPLIT ? 0 : im);
     for (int e0 = lane; e0 - lane < n * NCR; e0 += kU * 32) {
-        int at[kU];
         unsigned char fl[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int i = min((e0 + u * 32) / NCR, n - 1);
-            at[u] = row[i];
-            fl[u] = a.out[i];
-        }
+        for (int u = 0; u < kU; ++u) fl[u] = a.out[min((e0 + u * 32) / NCR, n - 1)];
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             const int i = min((e0 + u * 32) / NCR, n - 1);
-            R v = y[at[u] * NCR + comp];
+            R v = y[i * NCR + comp];
             if constexpr (NC == 1) {
                 if (e0 + u * 32 < n) io_store<double, IO>(a.io, sys, n, i, v);
             } else {
@@ -554,8 +562,22 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_con
     }
 }
 
-template <class R, int NCR, int IO>
-static void launch_flow(const std::vector<FlowJob>& jobs, cudaStream_t st) {
+template <class R, int IO>
+__global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow(const __grid_constant__ FlowMulti ms, int smem_sys) {
+    int bk = 0;
+    while (bk + 1 < ms.nb && (int)blockIdx.x >= ms.start[bk + 1]) ++bk;
+    const FlowArgs& a = ms.a[bk];
+    const int block = (int)blockIdx.x - ms.start[bk];
+    if (a.ncr == 4) flow_body<R, 4, IO>(a, block, smem_sys);
+    else flow_body<R, 2, IO>(a, block, smem_sys);
+}
+template <int IO>
+__global__ void __launch_bounds__(32 * kFlowWarps) k_solve_flow_real(const __grid_constant__ FlowMulti ms, int smem_sys) {
+    flow_body<double, 1, IO>(ms.a[0], (int)blockIdx.x, smem_sys);
+}
+
+template <class R, class Kernel>
+static void launch_flow(const std::vector<FlowJob>& jobs, Kernel kernel, cudaStream_t st) {
     if (jobs.size() > (size_t)kMaxGrp) throw InvalidArgument("scheduled solve: at most 8 handles per launch");
     constexpr int V = sizeof(R) == 8 ? 0 : 1;
     FlowMulti ms{};
@@ -564,7 +586,7 @@ static void launch_flow(const std::vector<FlowJob>& jobs, cudaStream_t st) {
     int systems = 0;
     for (const auto& j : jobs) {
         if (!j.form->data[V]) throw InvalidArgument("scheduled solve: call cng_banded_make_fp32 first");
-        smem = std::max(smem, flow_smem(j.form->rows, NCR, (int)sizeof(R)));
+        smem = std::max(smem, flow_smem(j.form->rows, j.form->ncr, (int)sizeof(R)));
         systems += j.s1 - j.s0;
     }
     // systems of a block: the count that keeps the most warps resident on an SM, where there are that many
@@ -576,39 +598,25 @@ static void launch_flow(const std::vector<FlowJob>& jobs, cudaStream_t st) {
     for (int k = 0; k < ms.nb; ++k) {
         const FlowForm& f = *jobs[k].form;
         ms.start[k] = total;
-        ms.a[k] = FlowArgs{f.n, f.rows, f.batch, jobs[k].s0, jobs[k].s1, f.sb[V], f.data[V], f.nchunk, f.perm, f.row,
+        ms.a[k] = FlowArgs{f.n, f.rows, f.ncr, f.batch, jobs[k].s0, jobs[k].s1, f.sb[V], f.data[V], f.nchunk, f.perm, f.row,
                            f.flags, f.flags + f.n, jobs[k].io, jobs[k].io2};
         total += ceil_div(jobs[k].s1 - jobs[k].s0, per);
     }
     ms.start[ms.nb] = total;
     if (total <= 0) return;
-    ensure_smem_attr((const void*)k_solve_flow<R, NCR, IO>, (int)kFlowSmem);
-    k_solve_flow<R, NCR, IO><<<total, 32 * per, smem * per, st>>>(ms, (int)smem);
+    ensure_smem_attr((const void*)kernel, (int)kFlowSmem);
+    kernel<<<total, 32 * per, smem * per, st>>>(ms, (int)smem);
     CNG_LAUNCH("k_solve_flow");
 }
 
 template <int IO>
 static void flow_io(const std::vector<FlowJob>& jobs, cudaStream_t st) {
-    // the handles of a launch have the same number of right-hand sides per factor
-    bool same = true;
-    for (const auto& j : jobs) same = same && j.form->ncr == jobs[0].form->ncr;
-    if (!same) {
-        for (int ncr : {4, 2, 1}) {
-            std::vector<FlowJob> part;
-            for (const auto& j : jobs)
-                if (j.form->ncr == ncr) part.push_back(j);
-            if (!part.empty()) flow_io<IO>(part, st);
-        }
-        return;
-    }
-    using R = std::conditional_t<IO == IO_MIXED, float, double>;
-    switch (jobs[0].form->ncr) {
-        case 1:
-            if constexpr (IO == IO_PLAIN || IO == IO_MAPPED) launch_flow<R, 1, IO>(jobs, st);
-            else throw InvalidArgument("solve_split needs complex (complex128) factors");
-            break;
-        case 2: launch_flow<R, 2, IO>(jobs, st); break;
-        default: launch_flow<R, 4, IO>(jobs, st); break;
+    if (jobs[0].form->dtype == 0) {
+        if constexpr (IO == IO_PLAIN || IO == IO_MAPPED) launch_flow<double>(jobs, k_solve_flow_real<IO>, st);
+        else throw InvalidArgument("solve_split needs complex (complex128) factors");
+    } else {
+        using R = std::conditional_t<IO == IO_MIXED, float, double>;
+        launch_flow<R>(jobs, k_solve_flow<R, IO>, st);
     }
 }
 

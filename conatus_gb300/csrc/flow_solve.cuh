@@ -38,7 +38,7 @@ struct FlowForm {
     size_t sb[2] = {0, 0};               // bytes of a system: FP64, FP32
     unsigned char* data[2] = {nullptr, nullptr};
     int* nchunk = nullptr;               // per system
-    unsigned short* row = nullptr;       // [batch][n]: the row of each column
+    unsigned short* row = nullptr;       // [batch][n]: the name of each row
     const int* perm = nullptr;           // NULL: the rows as they come
     unsigned char* flags = nullptr;      // [2][n]: rows' and columns' phase | partner's sign << 1
     ~FlowForm();
