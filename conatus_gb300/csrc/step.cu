@@ -202,17 +202,14 @@ __device__ __forceinline__ void split_residual_body(unsigned bid, unsigned nblk,
     for (unsigned w = (bid * blockDim.x + threadIdx.x) >> 5; w < nwarps; w += wstride) {
         const int i = (int)(w / sysw);
         const unsigned ml = (w - (unsigned)i * sysw) * 32u + lane;
-        if (ml >= (unsigned)cnt) continue;
-        const unsigned m = ml + (unsigned)s0;
+        const bool live = ml < (unsigned)cnt;                // the others run along (system s0's data, no store)
+        const unsigned m = (live ? ml : 0u) + (unsigned)s0;
         const long long t = (long long)m * n + i;
         const double2* xm = x + (long long)m * n;
         const double* mv = mono + (long long)m * nmono;
         const double2 bv = b[t];                            // in flight during the row's entries
         double ar = 0.0, ai = 0.0;
         const int e0 = ptr[i], e1 = ptr[i + 1];
-        // one pass over the row's entries (no data-dependent inner loop, so the loads of the next
-        // entries issue ahead); a term's group sum joins ar, ai when the term changes, as in the
-        // group-by-group order
         auto scale = [&](int tt) {
             // c = 1: no multiply; a merged list: its scale per (row, system) (NaN without the table)
             return tt == kMergedTerm ? (rowscale ? rowscale[(size_t)i * nsys + m] : __longlong_as_double(0x7ff8000000000000LL))
@@ -220,29 +217,53 @@ __device__ __forceinline__ void split_residual_body(unsigned bid, unsigned nblk,
         };
         int tt = e0 < e1 ? code[e0] >> 1 : 0;
         double gr = 0.0, gi = 0.0;
-#pragma unroll 4
-        for (int e = e0; e < e1; ++e) {
-            const int cd = code[e];
-            if ((cd >> 1) != tt) {
-                const double sc = scale(tt);
-                ar = fma(sc, gr, ar);
-                ai = fma(sc, gi, ai);
-                gr = gi = 0.0;
-                tt = cd >> 1;
+        // The entries of a row 32 at a time, one per lane, and x for kX of them in flight while the kX
+        // before are summed: the border rows' chains (n / 2 and more entries) waited for each entry's
+        // column, value and x in turn (RB 256 x 64: 29 us). A term's group sum joins ar, ai when the
+        // term changes, as in the group-by-group order
+        constexpr int kX = 4;
+        for (int eb = e0; eb < e1; eb += 32) {
+            const int nb = min(32, e1 - eb), el = eb + min((int)lane, nb - 1);
+            const int cl = col[el], cdl = code[el];
+            const double vl = val[el];
+            auto fetch = [&](double2* xv, int k0) {
+#pragma unroll
+                for (int u = 0; u < kX; ++u) {
+                    // x row-major over the systems when given: the warp's 32 systems read one line
+                    const int q = __shfl_sync(0xffffffffu, cl, min(k0 + u, nb - 1));
+                    xv[u] = xT ? xT[(size_t)q * nsys + m] : xm[q];
+                }
+            };
+            double2 cur[kX], nxt[kX];
+            fetch(cur, 0);
+            for (int k0 = 0; k0 < nb; k0 += kX) {
+                if (k0 + kX < nb) fetch(nxt, k0 + kX);
+#pragma unroll
+                for (int u = 0; u < kX; ++u) {
+                    if (k0 + u >= nb) break;
+                    const int cd = __shfl_sync(0xffffffffu, cdl, k0 + u);
+                    const double v = __shfl_sync(0xffffffffu, vl, k0 + u);
+                    if ((cd >> 1) != tt) {
+                        const double sc = scale(tt);
+                        ar = fma(sc, gr, ar);
+                        ai = fma(sc, gi, ai);
+                        gr = gi = 0.0;
+                        tt = cd >> 1;
+                    }
+                    const bool im = cd & 1;                  // i v x
+                    gr = fma(im ? -v : v, im ? cur[u].y : cur[u].x, gr);
+                    gi = fma(v, im ? cur[u].x : cur[u].y, gi);
+                }
+#pragma unroll
+                for (int u = 0; u < kX; ++u) cur[u] = nxt[u];
             }
-            const double v = val[e];
-            // x row-major over the systems when given: the warp's 32 systems read one line
-            const double2 xv = xT ? xT[(size_t)col[e] * nsys + m] : xm[col[e]];
-            const bool im = cd & 1;                          // i v x
-            gr = fma(im ? -v : v, im ? xv.y : xv.x, gr);
-            gi = fma(v, im ? xv.x : xv.y, gi);
         }
         if (e0 < e1) {
             const double sc = scale(tt);
             ar = fma(sc, gr, ar);
             ai = fma(sc, gi, ai);
         }
-        r[t] = make_double2(bv.x - ar, bv.y - ai);
+        if (live) r[t] = make_double2(bv.x - ar, bv.y - ai);
     }
 }
 
