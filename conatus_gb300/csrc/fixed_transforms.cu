@@ -6,7 +6,7 @@
 // What bounds them: 32 x 32 -> 64-bit products (12 per clock and SM) and the integer additions and
 // conversions beside them; the FP64 transforms they replace kept the FP64 pipe 85 % busy. Measured on the
 // channel 192 x 129 x 192 (x backward: 12 fields of 57600 columns, 96 modes -> 288 points, 2.65 GB):
-// 5.5 -> 1.84 ms; the whole right-hand side 14.7 -> 6.2 ms.
+// 5.5 -> 1.57 ms; the whole right-hand side 14.7 -> 5.0 ms.
 //
 // A column that holds a NaN or an infinity comes out as NaN throughout (a transform mixes every entry
 // into every output); zeros, denormals and the largest exponents are kept.
@@ -406,21 +406,24 @@ __device__ __forceinline__ void fx_cheb_body(unsigned bid, const FxChebArgs& a) 
     }
 }
 
+// 64 registers: these kernels wait on shared memory and on the products' latency, so resident warps count
+// for more than a few spilled words. Channel 192 x 129 x 192 right-hand side by blocks of 256 threads an
+// SM has registers for: 2 5.98 ms, 3 5.21, 4 5.03, 5 5.27; the ragged transforms 531, 483, 456, 471 us.
 template <bool REAL, bool FWD>
-__global__ void __launch_bounds__(kFxThreads, 2) k_fx_axis(const __grid_constant__ FxAxisArgs a) {
+__global__ void __launch_bounds__(kFxThreads, 4) k_fx_axis(const __grid_constant__ FxAxisArgs a) {
     fx_axis_body<REAL, FWD>(blockIdx.x, a);
 }
 template <bool REAL, bool FWD>
-__global__ void __launch_bounds__(kFxThreads, 2) k_fx_axis_grp(const __grid_constant__ Grp<FxAxisArgs> g) {
+__global__ void __launch_bounds__(kFxThreads, 4) k_fx_axis_grp(const __grid_constant__ Grp<FxAxisArgs> g) {
     const int k = g.find(blockIdx.x);
     fx_axis_body<REAL, FWD>(blockIdx.x - g.start[k], g.a[k]);
 }
 template <bool FWD>
-__global__ void __launch_bounds__(kFxThreads, 2) k_fx_cheb(const __grid_constant__ FxChebArgs a) {
+__global__ void __launch_bounds__(kFxThreads, 4) k_fx_cheb(const __grid_constant__ FxChebArgs a) {
     fx_cheb_body<FWD>(blockIdx.x, a);
 }
 template <bool FWD>
-__global__ void __launch_bounds__(kFxThreads, 2) k_fx_cheb_grp(const __grid_constant__ Grp<FxChebArgs> g) {
+__global__ void __launch_bounds__(kFxThreads, 4) k_fx_cheb_grp(const __grid_constant__ Grp<FxChebArgs> g) {
     const int k = g.find(blockIdx.x);
     fx_cheb_body<FWD>(blockIdx.x - g.start[k], g.a[k]);
 }
