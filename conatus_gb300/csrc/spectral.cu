@@ -523,6 +523,47 @@ __device__ __forceinline__ void cheb_der_warp(const c2<R>* __restrict__ c, c2<R>
     }
 }
 
+// The same with a lane per (eighth of the orders, parity, component) instead of a chunk of both parities
+// and components per lane: a sum takes N / 16 + 3 + N / 16 FP64 warp instructions instead of some 50
+// (each holds its sub-partition's unit for 64 cycles whatever its active lanes). Other partial sums, so
+// not where their roundings have to stay (launch_cheb). `two_k`: 2 k as doubles (converting an integer
+// is an FP64 instruction too).
+__device__ __forceinline__ void cheb_der_lanes(const double2* __restrict__ c, double2* __restrict__ der, int N,
+                                               const double* __restrict__ two_k, int lane) {
+    const int comp = lane & 1, par = (lane >> 1) & 1, seg = lane >> 2;
+    // orders k = par + 2 t, t in [t0, t1); par = 0 leaves out k = 0
+    const int T = (N - par + 1) >> 1, C = (T + 7) >> 3;
+    const int t0 = max(seg * C, par == 0 ? 1 : 0), t1 = min(seg * C + C, T);
+    const double* cc = reinterpret_cast<const double*>(c) + comp;
+    double* dd = reinterpret_cast<double*>(der) + comp;
+    double s = 0.0;
+    for (int t = t1 - 1; t >= t0; --t) {
+        const int k = par + 2 * t;
+        s = fma(two_k[k], cc[2 * k], s);
+    }
+    // the sums of the segments above this one
+    double a = __shfl_down_sync(0xffffffffu, s, 4);
+    if (seg == 7) a = 0.0;
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+        const double u = __shfl_down_sync(0xffffffffu, a, off);
+        if (lane + off < 32) a += u;
+    }
+    if (lane < 2) dd[2 * (N - 1)] = 0.0;
+    for (int t = t1 - 1; t >= t0; --t) {
+        const int k = par + 2 * t;
+        a = fma(two_k[k], cc[2 * k], a);
+        dd[2 * (k - 1)] = a;
+    }
+}
+
+// v 2^s, exact: on the exponent where v and the result are normal (no FP64 instruction)
+__device__ __forceinline__ double scale2(double v, int s) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    if (e == 0 || e == 0x7ff || e + s <= 0 || e + s >= 0x7ff) return v == 0.0 ? v : ldexp(v, s);
+    return __hiloint2double(hi + (s << 20), __double2loint(v));
+}
+
 // Arguments of the per-bucket stages (unpack, pack; a grouped launch holds one set per bucket).
 template <class R>
 struct BucketArgs {
@@ -542,8 +583,8 @@ __device__ __forceinline__ void unpack_body(unsigned bid, const RhsDev& d, const
     const int nw = blockDim.x >> 5;
     const int q = bid * nw + wib;
     const int m = q / split, part = q - m * split;      // system, and its y-groups part, part + split, ...
-    if (m >= b.nsys) return;
     const int Ny = d.Ny;
+    if (m >= b.nsys) return;
     // the system's state, rounded once to the transform precision R
     c2<R>* x = reinterpret_cast<c2<R>*>(sm) + (size_t)wib * (b.n + 2 * Ny);
     c2<R>* col = x + b.n;
@@ -616,6 +657,72 @@ __device__ __forceinline__ void unpack_body(unsigned bid, const RhsDev& d, const
     }
 }
 
+// FP64 with Fourier directions: a block per system, a warp per y-group, the state staged once. The warps
+// that each staged a system's whole state were few (16 an SM), and FP64 instructions bound them (scans of
+// the derivative, scaling by powers of two): channel 192 x 129 x 192 490 -> 254 us.
+__device__ __forceinline__ void unpack64_body(unsigned m, const RhsDev& d, const BucketDev& b,
+                                              const double2* __restrict__ state, double2* __restrict__ S) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int Ny = d.Ny;
+    double2* x = reinterpret_cast<double2*>(sm);
+    double2* col = x + b.n + (size_t)wib * 2 * Ny;
+    double* two_k = reinterpret_cast<double*>(x + b.n + (size_t)nw * 2 * Ny);
+    const double2* src = state + b.offset + (long long)m * b.n;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < b.n; i += blockDim.x) x[i] = src[i];
+    for (int k = threadIdx.x; k < Ny; k += blockDim.x) two_k[k] = 2.0 * k;
+    __syncthreads();
+    const int jx = b.modes[2 * m], jz = b.modes[2 * m + 1];
+    const int slot = zslot(jz, b.sign, d.Nzc);
+    const int cbase = (b.case_of ? b.case_of[m] : 0) * d.ngy;
+    // the amplitude scale is a power of two, and so is 2 / L on most intervals
+    const double sc = 2.0 / d.ly;
+    const bool pow2 = ((__double2hiint(sc) & 0xfffff) | __double2loint(sc)) == 0;
+    const int sc2 = (__double2hiint(sc) >> 20) - 1023;
+    for (int gy = wib; gy < d.ngy; gy += nw) {
+        const int f = d.yg_rep[gy], oy = d.factors[5 * f + 3];
+        const int* cp = b.colpos + (size_t)f * Ny;
+        const long long fc = cbase + gy;
+        double2* dst = S + (d.ndir == 2 ? (fc * d.Kx + jx) * d.Nzc + slot : fc * d.Kx + jx) * Ny;
+        double2* dstc = d.ndir == 2 && jx == 0 && jz > 0 ? S + (fc * d.Kx * d.Nzc + (d.Nzc - jz)) * Ny : nullptr;
+        auto store = [&](int nn, double2 v) {
+            v.x = scale2(v.x, -b.dact);
+            v.y = b.real ? 0.0 : scale2(v.y, -b.dact);
+            dst[nn] = v;
+            if (dstc) dstc[nn] = make_double2(v.x, -v.y);
+        };
+        double2 *from = col, *to = col + Ny;
+#pragma unroll 4
+        for (int nn = lane; nn < Ny; nn += 32) {
+            const int pos = cp[nn];
+            const double2 v = pos >= 0 ? x[pos] : make_double2(0.0, 0.0);
+            if (oy == 0) store(nn, v);
+            else from[nn] = v;
+        }
+        __syncwarp();
+        for (int rep = 0; rep < oy; ++rep) {
+            cheb_der_lanes(from, to, Ny, two_k, lane);
+            __syncwarp();
+#pragma unroll 4
+            for (int nn = lane; nn < Ny; nn += 32) {
+                double2 v = to[nn];
+                const int h = nn == 0 ? -1 : 0;
+                if (pow2) {
+                    v.x = scale2(v.x, sc2 + h);
+                    v.y = scale2(v.y, sc2 + h);
+                } else {
+                    v.x = scale2(v.x, h) * sc;
+                    v.y = scale2(v.y, h) * sc;
+                }
+                if (rep + 1 < oy) from[nn] = v;
+                else store(nn, v);
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // every bucket of one or more evaluators in one launch (launch_unpack)
 template <class R>
 __global__ void k_unpack_grp(const __grid_constant__ Grp<BucketArgs<R>> g) {
@@ -623,6 +730,11 @@ __global__ void k_unpack_grp(const __grid_constant__ Grp<BucketArgs<R>> g) {
     const BucketArgs<R>& a = g.a[k];
     unpack_body<R>(blockIdx.x - g.start[k], a.d, a.b, static_cast<const double2*>(a.in), static_cast<c2<R>*>(a.out),
                    a.split);
+}
+__global__ void k_unpack64_grp(const __grid_constant__ Grp<BucketArgs<double>> g) {
+    const int k = g.find(blockIdx.x);
+    const BucketArgs<double>& a = g.a[k];
+    unpack64_body(blockIdx.x - g.start[k], a.d, a.b, static_cast<const double2*>(a.in), static_cast<double2*>(a.out));
 }
 
 // products on the grid: out_o = sum_m c_m prod_j G_j. The monomial tables are staged in shared
@@ -1129,6 +1241,32 @@ static void launch_unpack(Rhs* const* hs, int n, const double2* state, cudaStrea
     size_t smem = 0;
     int ngy = 1;
     for (int i = 0; i < n; ++i) ngy = std::max(ngy, hs[i]->dev.ngy);
+    if constexpr (sizeof(R) == 8) {
+        bool shared = true;
+        for (int i = 0; i < n; ++i) shared = shared && hs[i]->dev.share && hs[i]->ndir > 0;
+        auto bytes = [&](int nw) {
+            size_t most = 0;
+            for (int i = 0; i < n; ++i)
+                for (const auto& b : hs[i]->buckets)
+                    most = std::max(most, ((size_t)b.n + 2 * (size_t)nw * hs[i]->ny) * sizeof(double2) + (size_t)hs[i]->ny * sizeof(double));
+            return most;
+        };
+        int nw = std::min(ngy, 8);
+        while (nw > 1 && bytes(nw) > 200 * 1024) --nw;
+        if (shared && bytes(nw) <= 200 * 1024) {
+            for (int i = 0; i < n; ++i)
+                for (const auto& b : hs[i]->buckets) {
+                    args.push_back(BucketArgs<R>{hs[i]->dev, b, state, hs[i]->S, 1});
+                    blocks.push_back((unsigned)b.nsys);
+                }
+            ensure_smem_attr((const void*)k_unpack64_grp, 200 * 1024);
+            launch_groups(args, blocks, [&](const Grp<BucketArgs<R>>& g, unsigned total) {
+                k_unpack64_grp<<<total, 32 * nw, bytes(nw), st>>>(g);
+                CNG_LAUNCH("k_unpack64_grp");
+            });
+            return;
+        }
+    }
     const int split = bucket_split(hs, n, std::min(ngy, 8));
     for (int i = 0; i < n; ++i)
         for (const auto& b : hs[i]->buckets) {
