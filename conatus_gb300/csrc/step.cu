@@ -184,8 +184,14 @@ __global__ void k_poly_residual(int nsys, int n, const int* __restrict__ ip, con
 // a dozen) and the entry data is one broadcast load per warp; x is gathered per lane.
 constexpr int kMergedTerm = 63;          // an entry list shared by several terms: scale per (row, system)
 
-// Systems s0 .. s0 + cnt - 1 of a bucket of ld systems (rowscale and xT are [n][ld]).
-template <bool CONE>
+// -v where im, on the sign bit (no FP64 instruction)
+__device__ __forceinline__ double neg_if(double v, bool im) {
+    return __hiloint2double(__double2hiint(v) ^ (im ? (int)0x80000000 : 0), __double2loint(v));
+}
+
+// Systems s0 .. s0 + cnt - 1 of a bucket of ld systems (rowscale and xT are [n][ld]). XT: x comes row-major
+// over the systems (many systems, FP64 bound: a plain loop over the entries keeps its pipe busiest).
+template <bool CONE, bool XT>
 __device__ __forceinline__ void split_residual_body(unsigned bid, unsigned nblk, int cnt, int s0, int ld, int n,
                                                     const int* __restrict__ ptr, const int* __restrict__ col,
                                                     const double* __restrict__ val,
@@ -217,45 +223,51 @@ __device__ __forceinline__ void split_residual_body(unsigned bid, unsigned nblk,
         };
         int tt = e0 < e1 ? code[e0] >> 1 : 0;
         double gr = 0.0, gi = 0.0;
-        // The entries of a row 32 at a time, one per lane, and x for kX of them in flight while the kX
-        // before are summed: the border rows' chains (n / 2 and more entries) waited for each entry's
-        // column, value and x in turn (RB 256 x 64: 29 us). A term's group sum joins ar, ai when the
-        // term changes, as in the group-by-group order
-        constexpr int kX = 4;
-        for (int eb = e0; eb < e1; eb += 32) {
-            const int nb = min(32, e1 - eb), el = eb + min((int)lane, nb - 1);
-            const int cl = col[el], cdl = code[el];
-            const double vl = val[el];
-            auto fetch = [&](double2* xv, int k0) {
+        // a term's group sum joins ar, ai when the term changes, as in the group-by-group order
+        auto entry = [&](int cd, double v, double2 xv) {
+            if ((cd >> 1) != tt) {
+                const double sc = scale(tt);
+                ar = fma(sc, gr, ar);
+                ai = fma(sc, gi, ai);
+                gr = gi = 0.0;
+                tt = cd >> 1;
+            }
+            const bool im = cd & 1;                          // i v x
+            gr = fma(neg_if(v, im), im ? xv.y : xv.x, gr);
+            gi = fma(v, im ? xv.x : xv.y, gi);
+        };
+        if constexpr (XT) {
+            // the warp's 32 systems read one line; the next entries' loads issue ahead
+#pragma unroll 4
+            for (int e = e0; e < e1; ++e) entry(code[e], val[e], xT[(size_t)col[e] * nsys + m]);
+        } else {
+            // The entries of a row 32 at a time, one per lane, and x for kX of them in flight while the kX
+            // before are summed: the border rows' chains (n / 2 and more entries) waited for each entry's
+            // column, value and x in turn (RB 256 x 64: 29 -> 26 us)
+            constexpr int kX = 4;
+            for (int eb = e0; eb < e1; eb += 32) {
+                const int nb = min(32, e1 - eb), el = eb + min((int)lane, nb - 1);
+                const int cl = col[el], cdl = code[el];
+                const double vl = val[el];
+                auto fetch = [&](double2* xv, int k0) {
 #pragma unroll
-                for (int u = 0; u < kX; ++u) {
-                    // x row-major over the systems when given: the warp's 32 systems read one line
-                    const int q = __shfl_sync(0xffffffffu, cl, min(k0 + u, nb - 1));
-                    xv[u] = xT ? xT[(size_t)q * nsys + m] : xm[q];
-                }
-            };
-            double2 cur[kX], nxt[kX];
-            fetch(cur, 0);
-            for (int k0 = 0; k0 < nb; k0 += kX) {
-                if (k0 + kX < nb) fetch(nxt, k0 + kX);
-#pragma unroll
-                for (int u = 0; u < kX; ++u) {
-                    if (k0 + u >= nb) break;
-                    const int cd = __shfl_sync(0xffffffffu, cdl, k0 + u);
-                    const double v = __shfl_sync(0xffffffffu, vl, k0 + u);
-                    if ((cd >> 1) != tt) {
-                        const double sc = scale(tt);
-                        ar = fma(sc, gr, ar);
-                        ai = fma(sc, gi, ai);
-                        gr = gi = 0.0;
-                        tt = cd >> 1;
+                    for (int u = 0; u < kX; ++u) {
+                        const int q = __shfl_sync(0xffffffffu, cl, min(k0 + u, nb - 1));
+                        xv[u] = xT ? xT[(size_t)q * nsys + m] : xm[q];
                     }
-                    const bool im = cd & 1;                  // i v x
-                    gr = fma(im ? -v : v, im ? cur[u].y : cur[u].x, gr);
-                    gi = fma(v, im ? cur[u].x : cur[u].y, gi);
-                }
+                };
+                double2 cur[kX], nxt[kX];
+                fetch(cur, 0);
+                for (int k0 = 0; k0 < nb; k0 += kX) {
+                    if (k0 + kX < nb) fetch(nxt, k0 + kX);
 #pragma unroll
-                for (int u = 0; u < kX; ++u) cur[u] = nxt[u];
+                    for (int u = 0; u < kX; ++u) {
+                        if (k0 + u >= nb) break;
+                        entry(__shfl_sync(0xffffffffu, cdl, k0 + u), __shfl_sync(0xffffffffu, vl, k0 + u), cur[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kX; ++u) cur[u] = nxt[u];
+                }
             }
         }
         if (e0 < e1) {
@@ -275,15 +287,15 @@ __global__ void k_split_residual(int cnt, int s0, int ld, int n, const int* __re
                                  const double* __restrict__ rowscale, const double2* __restrict__ x,
                                  const double2* __restrict__ xT, const double2* __restrict__ b,
                                  double2* __restrict__ r) {
-    split_residual_body<CONE>(blockIdx.x, gridDim.x, cnt, s0, ld, n, ptr, col, val, code, mono, nmono, a, c,
+    split_residual_body<CONE, false>(blockIdx.x, gridDim.x, cnt, s0, ld, n, ptr, col, val, code, mono, nmono, a, c,
                               rowscale, x, xT, b, r);
 }
 
-template <bool CONE>
+template <bool CONE, bool XT>
 __global__ void k_split_residual_grp(const __grid_constant__ Grp<cng_residual_part> g, double a, double c) {
     const int k = g.find(blockIdx.x);
     const cng_residual_part& p = g.a[k];
-    split_residual_body<CONE>(blockIdx.x - g.start[k], g.start[k + 1] - g.start[k], p.s1 - p.s0, p.s0, p.nsys, p.n,
+    split_residual_body<CONE, XT>(blockIdx.x - g.start[k], g.start[k + 1] - g.start[k], p.s1 - p.s0, p.s0, p.nsys, p.n,
                               p.ptr, p.col, p.val, reinterpret_cast<const signed char*>(p.code), p.mono, p.nmono, a, c,
                               p.rowscale, static_cast<const double2*>(p.x), static_cast<const double2*>(p.xT),
                               static_cast<const double2*>(p.b), static_cast<double2*>(p.r));
@@ -367,8 +379,11 @@ int cng_split_residual_group(int nparts, const cng_residual_part* parts, double 
         }
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         launch_groups(args, blocks, [&](const Grp<cng_residual_part>& g, unsigned total) {
-            if (c == 1.0) k_split_residual_grp<true><<<total, 256, 0, st>>>(g, a, c);
-            else k_split_residual_grp<false><<<total, 256, 0, st>>>(g, a, c);
+            bool xt = true;
+            for (int k = 0; k < g.n; ++k) xt = xt && g.a[k].xT;
+            const auto kernel = xt ? (c == 1.0 ? k_split_residual_grp<true, true> : k_split_residual_grp<false, true>)
+                                   : (c == 1.0 ? k_split_residual_grp<true, false> : k_split_residual_grp<false, false>);
+            kernel<<<total, 256, 0, st>>>(g, a, c);
             CNG_LAUNCH("k_split_residual_grp");
         });
     })
