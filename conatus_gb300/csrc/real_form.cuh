@@ -20,11 +20,12 @@ __device__ __forceinline__ double real_part_of(zd v, int dp, int& bad) {
     if ((imag ? v.re : v.im) != 0.0) bad = 1;
     return imag ? (dp > 0 ? v.im : -v.im) : v.re;
 }
+// -v on the sign bit: an FP64 negation is an instruction of the FP64 unit
+__device__ __forceinline__ double flip(double v) { return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v)); }
+__device__ __forceinline__ float flip(float v) { return -v; }
 // i^-p b and i^q x
 template <class T>
-__device__ __forceinline__ T phase_in(T b, int p) { return p ? T(b.im, -b.re) : b; }
-template <class T>
-__device__ __forceinline__ T phase_out(T x, int q) { return q ? T(-x.im, x.re) : x; }
+__device__ __forceinline__ T phase_in(T b, int p) { return p ? T(b.im, flip(b.re)) : b; }
 
 // Row and column phases of the assembled systems (band `ab` and border rows `vt`, before the
 // factorization), found on up to 256 of them; false where there are none. What is built from the
