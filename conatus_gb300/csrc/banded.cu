@@ -730,9 +730,6 @@ struct Banded {
     unsigned char* rowp = nullptr;
     unsigned char* colp = nullptr;
     std::unique_ptr<FlowForm> flow;
-    // host solves: one device buffer for the right-hand sides, made by the first of them; calls take turns
-    std::mutex host_turn;
-    void* host_buf = nullptr;
     // shared-pattern refactorization data (create_shared)
     int nnz = 0;
     long long* bulk_dest = nullptr;
@@ -746,7 +743,7 @@ struct Banded {
                         (void*)bp, (void*)bcol, (void*)ab32, (void*)vt32, (void*)w32, (void*)slu32,
                         (void*)c_offL, (void*)c_Lrow, (void*)c_Lmask, (void*)c_offU, (void*)c_Udist,
                         (void*)c_offV, (void*)c_Vcol, c_L, c_U, c_V, (void*)c_piv, (void*)c_L32,
-                        (void*)c_U32, (void*)c_V32, (void*)flip_r, (void*)flip_c, p_Rf, p_Rb, w_scr, host_buf, (void*)rowp,
+                        (void*)c_U32, (void*)c_V32, (void*)flip_r, (void*)flip_c, p_Rf, p_Rb, w_scr, (void*)rowp,
                         (void*)colp})
             dev_free(p);
     }
@@ -1346,22 +1343,26 @@ int cng_banded_solve_host(cng_banded* hh, const void* b_host, void* x_host, int 
         Banded* h = as_banded(hh);
         if (!b_host || !x_host) throw InvalidArgument("BorderedBandedBatch.solve: null host pointer");
         const size_t bytes = h->esz * (size_t)h->batch * h->n;
+        void* d = nullptr;
         cudaStream_t st = nullptr;
-        std::lock_guard<std::mutex> turn(h->host_turn);
-        // kept with the handle: allocating and freeing it took 20 of a call's 52 us (31 systems, n = 270)
-        if (!h->host_buf) h->host_buf = dev_alloc(bytes);
-        void* d = h->host_buf;
-        CNG_CUDA(cudaMemcpyAsync(d, b_host, bytes, cudaMemcpyHostToDevice, st));
-        if (transpose) {
-            prepare_transpose(*h, st);
-            if (h->dtype == 0) launch_solve_T_t<double>(*h, d, st);
-            else launch_solve_T_t<zd>(*h, d, st);
-        } else {
-            SolveIo io{d, d, nullptr, nullptr, nullptr, nullptr};
-            launch_solve(*h, IO_PLAIN, io, st);
+        CNG_CUDA(cudaMalloc(&d, bytes));
+        try {
+            CNG_CUDA(cudaMemcpyAsync(d, b_host, bytes, cudaMemcpyHostToDevice, st));
+            if (transpose) {
+                prepare_transpose(*h, st);
+                if (h->dtype == 0) launch_solve_T_t<double>(*h, d, st);
+                else launch_solve_T_t<zd>(*h, d, st);
+            } else {
+                SolveIo io{d, d, nullptr, nullptr, nullptr, nullptr};
+                launch_solve(*h, IO_PLAIN, io, st);
+            }
+            CNG_CUDA(cudaMemcpyAsync(x_host, d, bytes, cudaMemcpyDeviceToHost, st));
+            CNG_CUDA(cudaStreamSynchronize(st));
+        } catch (...) {
+            cudaFree(d);
+            throw;
         }
-        CNG_CUDA(cudaMemcpyAsync(x_host, d, bytes, cudaMemcpyDeviceToHost, st));
-        CNG_CUDA(cudaStreamSynchronize(st));
+        CNG_CUDA(cudaFree(d));
     })
 }
 
