@@ -778,23 +778,22 @@ struct ProductArgs {
     long long P;
 };
 
-template <class R, int V>
-__device__ __forceinline__ void products_body(unsigned bid, unsigned nblk, const RhsDev& d, const R* __restrict__ G,
-                                              R* __restrict__ O, long long P) {
-    __shared__ int s_ptr[17];
-    __shared__ R s_coef[kMaxMono];
-    __shared__ int s_kind[kMaxMono];         // 1: coefficient +1, -1: coefficient -1, 0: other
-    __shared__ int s_fac[4 * kMaxMono];
+// v with its sign bit changed by `mask` (0 or 1 << 31): a negation is an FP64 instruction
+__device__ __forceinline__ double flip_by(double v, int mask) {
+    return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
+}
+__device__ __forceinline__ float flip_by(float v, int mask) { return __int_as_float(__float_as_int(v) ^ mask); }
+
+// What bounds it: an FP64 instruction per monomial and 32 points beside the HBM bytes of the factors and
+// outputs, each about 0.3 ms on the channel 192 x 129 x 192 (9 monomials, 15 fields of 16.6 M points).
+// Where every coefficient is +-1 and no monomial has more than two factors (SIMPLE; every committed problem)
+// the code holds no negation and no other product, which took a second instruction even where their
+// results were not used: 572 us there, 349 without it.
+template <class R, int V, bool SIMPLE>
+__device__ __forceinline__ void products_points(unsigned bid, unsigned nblk, const RhsDev& d, const R* __restrict__ G,
+                                                R* __restrict__ O, long long P, const int* s_ptr, const R* s_coef,
+                                                const int* s_sign, const int* s_fac) {
     const int no = d.noutputs;
-    for (int q = threadIdx.x; q <= no; q += blockDim.x) s_ptr[q] = d.out_mono_ptr[q];
-    __syncthreads();
-    const int nm = s_ptr[no];
-    for (int q = threadIdx.x; q < nm; q += blockDim.x) {
-        s_coef[q] = R(d.mono_coef[q]);
-        s_kind[q] = d.mono_coef[q] == 1.0 ? 1 : (d.mono_coef[q] == -1.0 ? -1 : 0);
-    }
-    for (int q = threadIdx.x; q < 4 * nm; q += blockDim.x) s_fac[q] = d.mono_fac[q];
-    __syncthreads();
     const long long total = P * d.ncase;
     for (long long t0 = ((long long)bid * blockDim.x + threadIdx.x) * V; t0 < total;
          t0 += (long long)nblk * blockDim.x * V) {
@@ -807,57 +806,59 @@ __device__ __forceinline__ void products_body(unsigned bid, unsigned nblk, const
             for (int v = 0; v < V; ++v) acc[v] = R(0);
             for (int mi = s_ptr[o]; mi < s_ptr[o + 1]; ++mi) {
                 // c G_a (G_b G_c G_d): the product of the later factors, then one fused
-                // multiply-add with the first factor times c (c = +-1: the sign goes into the
-                // fused multiply-add; the kind of c is read, not compared, per point)
-                const R cf = s_coef[mi];
-                const int kind = s_kind[mi];
-                R pr[V];
-                bool have = false;
+                // multiply-add with the first factor times c (SIMPLE: its sign bit)
+                R pr[V];                         // 1 where there is no later factor
 #pragma unroll
-                for (int q = 1; q < 4; ++q) {
-                    const int f = s_fac[4 * mi + q];
-                    if (f >= 0) {
+                for (int v = 0; v < V; ++v) pr[v] = R(1);
+                if (s_fac[4 * mi + 1] >= 0) load_v<R, V>(Gc + (long long)s_fac[4 * mi + 1] * P, pr);
+                if constexpr (!SIMPLE) {
+                    for (int q = 2; q < 4; ++q) {
+                        const int f = s_fac[4 * mi + q];
+                        if (f < 0) continue;
                         R g[V];
                         load_v<R, V>(Gc + (long long)f * P, g);
-                        if (have) {
 #pragma unroll
-                            for (int v = 0; v < V; ++v) pr[v] = pr[v] * g[v];
-                        } else {
-#pragma unroll
-                            for (int v = 0; v < V; ++v) pr[v] = g[v];
-                        }
-                        have = true;
+                        for (int v = 0; v < V; ++v) pr[v] = pr[v] * g[v];
                     }
                 }
                 const int f0 = s_fac[4 * mi];
                 R a[V];
                 if (f0 >= 0) {
                     load_v<R, V>(Gc + (long long)f0 * P, a);
-                    if (kind == 0) {
 #pragma unroll
-                        for (int v = 0; v < V; ++v) a[v] = cf * a[v];
-                    }
+                    for (int v = 0; v < V; ++v) a[v] = SIMPLE ? flip_by(a[v], s_sign[mi]) : s_coef[mi] * a[v];
                 } else {
 #pragma unroll
-                    for (int v = 0; v < V; ++v) a[v] = cf;
+                    for (int v = 0; v < V; ++v) a[v] = s_coef[mi];
                 }
-                if (have && f0 >= 0 && kind < 0) {
 #pragma unroll
-                    for (int v = 0; v < V; ++v) acc[v] = fmar(-a[v], pr[v], acc[v]);
-                } else if (have) {
-#pragma unroll
-                    for (int v = 0; v < V; ++v) acc[v] = fmar(a[v], pr[v], acc[v]);
-                } else if (f0 >= 0 && kind < 0) {
-#pragma unroll
-                    for (int v = 0; v < V; ++v) acc[v] = acc[v] - a[v];
-                } else {
-#pragma unroll
-                    for (int v = 0; v < V; ++v) acc[v] = acc[v] + a[v];
-                }
+                for (int v = 0; v < V; ++v) acc[v] = fmar(a[v], pr[v], acc[v]);
             }
             store_v<R, V>(Oc + (long long)o * P, acc);
         }
     }
+}
+
+template <class R, int V>
+__device__ __forceinline__ void products_body(unsigned bid, unsigned nblk, const RhsDev& d, const R* __restrict__ G,
+                                              R* __restrict__ O, long long P) {
+    __shared__ int s_ptr[17];
+    __shared__ R s_coef[kMaxMono];
+    __shared__ int s_sign[kMaxMono];         // the coefficient's sign bit
+    __shared__ int s_fac[4 * kMaxMono];
+    const int no = d.noutputs;
+    for (int q = threadIdx.x; q <= no; q += blockDim.x) s_ptr[q] = d.out_mono_ptr[q];
+    __syncthreads();
+    const int nm = s_ptr[no];
+    int other = 0;
+    for (int q = threadIdx.x; q < nm; q += blockDim.x) {
+        s_coef[q] = R(d.mono_coef[q]);
+        s_sign[q] = __double2hiint(d.mono_coef[q]) & (int)0x80000000;
+        other |= fabs(d.mono_coef[q]) != 1.0 || d.mono_fac[4 * q + 2] >= 0 || d.mono_fac[4 * q + 3] >= 0;
+    }
+    for (int q = threadIdx.x; q < 4 * nm; q += blockDim.x) s_fac[q] = d.mono_fac[q];
+    if (__syncthreads_or(other)) products_points<R, V, false>(bid, nblk, d, G, O, P, s_ptr, s_coef, s_sign, s_fac);
+    else products_points<R, V, true>(bid, nblk, d, G, O, P, s_ptr, s_coef, s_sign, s_fac);
 }
 
 template <class R, int V>
