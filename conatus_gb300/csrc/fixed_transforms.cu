@@ -6,7 +6,7 @@
 // What bounds them: 32 x 32 -> 64-bit products (12 per clock and SM) and the integer additions and
 // conversions beside them; the FP64 transforms they replace kept the FP64 pipe 85 % busy. Measured on the
 // channel 192 x 129 x 192 (x backward: 12 fields of 57600 columns, 96 modes -> 288 points, 2.65 GB):
-// 5.5 -> 1.57 ms; the whole right-hand side 14.7 -> 5.0 ms.
+// 5.5 -> 1.57 ms; the whole right-hand side 14.7 -> 5.0 ms (4.76 with the later products).
 //
 // A column that holds a NaN or an infinity comes out as NaN throughout (a transform mixes every entry
 // into every output); zeros, denormals and the largest exponents are kept.
@@ -61,7 +61,12 @@ struct FxCol {
         return !bad && fx_plain(b) ? fx_to(v, b) : fx_to_any(v, b, bad);
     }
 };
-__device__ __forceinline__ int fx_exponent(double d) { return fx_hiword(d) & 0x7ff00000; }
+// of a column's largest entry: the exponent from bit 20 on, and 0 for a column of zeros alone
+__device__ __forceinline__ int fx_magnitude(double d) { return (fx_hiword(d) & 0x7fffffff) | (fx_loword(d) ? 1 : 0); }
+// its exponent field. Zeros take that of 1, which keeps them (and fields that are not excited, or modes
+// whose derivative is zero) off the slow way back for the ends of the range: a right-hand side of a zero
+// state 9.5 ms on the channel 192 x 129 x 192 without this, 4.9 with it (a random state 4.8)
+__device__ __forceinline__ int fx_column(int magnitude) { return magnitude ? max(magnitude >> 20, 1) : 1023; }
 
 template <class Out, class Shift>
 __device__ __forceinline__ void fx_stages(fx2* z, const FxPlan& pl, int n, int lc, int CS, Out&& out, Shift&& shift) {
@@ -147,22 +152,21 @@ __device__ __forceinline__ void fx_axis_body(unsigned bid, const FxAxisArgs& a) 
 #pragma unroll
         for (int u = 0; u < H; ++u)
 #pragma unroll
-            for (int q = 0; q < NV; ++q) em = max(em, fx_exponent(held[u][q]));
+            for (int q = 0; q < NV; ++q) em = max(em, fx_magnitude(held[u][q]));
     } else {
         for (int e = tid; e < items; e += nt) {
             load(e, held[0]);
 #pragma unroll
-            for (int q = 0; q < NV; ++q) em = max(em, fx_exponent(held[0][q]));
+            for (int q = 0; q < NV; ++q) em = max(em, fx_magnitude(held[0][q]));
         }
     }
     __syncthreads();
     for (int m = C; m < 32; m <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, m));
     if (lane < C) atomicMax(&s_e[c], em);
     __syncthreads();
-    em = s_e[c] >> 20;
+    em = fx_column(s_e[c]);
     FxCol fc;
     fc.bad = em == 0x7ff;
-    em = max(em, 1);
     unsigned T = 0;
     if (hold) {
 #pragma unroll
@@ -316,18 +320,17 @@ __device__ __forceinline__ void fx_cheb_body(unsigned bid, const FxChebArgs& a) 
 #pragma unroll
             for (int u = 0; u < H; ++u)
 #pragma unroll
-                for (int q = 0; q < NV; ++q) em = max(em, fx_exponent(held[u][q]));
+                for (int q = 0; q < NV; ++q) em = max(em, fx_magnitude(held[u][q]));
         } else {
             for (int u = lane; u < items; u += 32) {
                 load(u, held[0]);
 #pragma unroll
-                for (int q = 0; q < NV; ++q) em = max(em, fx_exponent(held[0][q]));
+                for (int q = 0; q < NV; ++q) em = max(em, fx_magnitude(held[0][q]));
             }
         }
-        em = __reduce_max_sync(0xffffffffu, em) >> 20;
+        em = fx_column(__reduce_max_sync(0xffffffffu, em));
         FxCol fc;
         fc.bad = em == 0x7ff;
-        em = max(em, 1);
         if (hold) {
 #pragma unroll
             for (int u = 0; u < H; ++u)
