@@ -35,6 +35,7 @@ constexpr int kRing = 3;                         // chunks staged in shared memo
                                                  // 9, channel 128 x 129 x 128 351 us against 298)
 constexpr int kFlowWarps = 4;                    // most systems of a block
 constexpr size_t kFlowSmem = 220 * 1024;
+constexpr size_t kFlowLoose = 64 << 20;           // bytes of operations laid out at their most, uncounted
 constexpr int kMaxBorder = 64;
 constexpr unsigned kFresh = 0x80000000u;         // the operation's sum starts from 0
 
@@ -69,7 +70,7 @@ __device__ __forceinline__ bool pure_imag(zd v) { return v.re == 0.0 && v.im != 
 
 // The schedule of one system, by one warp. `ready` of a row: the slot after its last write; `read`: the
 // last slot that reads it (a slot reads before it writes).
-template <class R, bool COUNT>
+template <bool COUNT>
 struct FlowPlan {
     int *ready, *read;
     unsigned short* next;                        // where to look for room from a slot on
@@ -106,8 +107,8 @@ struct FlowPlan {
                 if constexpr (!COUNT) {
                     unsigned char* ch = data + (size_t)(t / kSlots) * chunk;
                     const int e = (t % kSlots) * ops + at + rank;
-                    reinterpret_cast<R*>(ch)[e] = (R)(-c);
-                    reinterpret_cast<unsigned*>(ch + (size_t)kSlots * ops * sizeof(R))[e] =
+                    reinterpret_cast<double*>(ch)[e] = -c;
+                    reinterpret_cast<unsigned*>(ch + (size_t)kSlots * ops * sizeof(double))[e] =
                         (unsigned)src | (unsigned)dst << 16 | (fresh ? kFresh : 0u);
                 }
                 open = false;
@@ -124,14 +125,18 @@ struct FlowPlan {
     }
 };
 
-// One warp per system. COUNT: its slots into nslot; else the operations (R: type of the values).
+// One warp per system: its slots into nslot and, unless COUNT, its operations.
 // stat[0]: not of the form, stat[1]: more slots than allowed.
-template <class T, class R, bool COUNT>
+// What bounds it: the latency of one warp, 1.7 ms for n = 522, whatever the number of systems. So a batch
+// whose operations fit 64 MB at their most is written without the counting pass, and the FP32 copies are
+// rounded from the others (a third pass before): factorization of channel 96 x 129 x 96 61 -> 57 ms, with FP32
+// copies 69 -> 59, of 128 host-built systems of n = 262 12.0 -> 10.5 ms (10.5 without the operations too).
+template <class T, bool COUNT>
 __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int* stat, FlowOut o) {
     extern __shared__ __align__(16) unsigned char fsm[];
     const int n = in.s.n, r = in.s.r, kl = in.s.kl, kv = in.kv, ldab = in.s.ldab, rows = in.rows, LS = in.s.lanes;
     const int sys = blockIdx.x, lane = threadIdx.x;
-    FlowPlan<R, COUNT> put;
+    FlowPlan<COUNT> put;
     put.ready = reinterpret_cast<int*>(fsm);
     put.read = put.ready + rows;
     unsigned short* ord = reinterpret_cast<unsigned short*>(put.read + rows);      // row at a position
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
     unsigned char* rowph = put.cnt + in.cap;
     put.data = COUNT ? nullptr : o.data + (size_t)sys * o.sb;
     put.ops = flow_ops(in.ncr);
-    put.chunk = flow_chunk(in.ncr, (int)sizeof(R));
+    put.chunk = flow_chunk(in.ncr, (int)sizeof(double));
     put.cap = in.cap;
     put.lane = lane;
     const T* ab = in.ab + (size_t)sys * n * ldab;
@@ -288,10 +293,8 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
                 put(v != 0.0, z(k), v != 0.0 ? j : 0, v, false);
             }
     }
-    if constexpr (COUNT) {
-        const int end = __reduce_max_sync(0xffffffffu, put.end);
-        if (lane == 0) nslot[sys] = end;
-    }
+    const int end = __reduce_max_sync(0xffffffffu, put.end);
+    if (lane == 0) nslot[sys] = end;
     if (bad) stat[0] = 1;
     if (put.over) stat[1] = 1;
 }
@@ -302,6 +305,18 @@ __global__ void k_flow_clear(unsigned char* data, size_t sb, int batch, int chun
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < per * batch; e += (size_t)gridDim.x * blockDim.x) {
         const size_t sys = e / per, w = e - sys * per;
         reinterpret_cast<unsigned*>(data + sys * sb)[w] = (int)(w % (chunk / 4)) * 4 < vbytes ? 0u : none;
+    }
+}
+
+// the FP32 copies: the same rows, the values rounded; `per` operations to a chunk
+__global__ void k_flow_demote(const unsigned char* __restrict__ in, unsigned char* __restrict__ out, long long total, int per) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+        const long long g = e / per;
+        const int i = (int)(e - g * per);
+        const unsigned char* a = in + g * per * 12;
+        unsigned char* b = out + g * per * 8;
+        reinterpret_cast<float*>(b)[i] = (float)reinterpret_cast<const double*>(a)[i];
+        reinterpret_cast<unsigned*>(b)[per + i] = reinterpret_cast<const unsigned*>(a)[2 * per + i];
     }
 }
 
@@ -342,9 +357,8 @@ static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
     const int cap = std::min(65000, kFlowColumnBytes * (n + 64) / (12 * ops) / kSlots * kSlots);
     const size_t smem = (size_t)f->rows * 8 + (size_t)n * 7 + (size_t)cap * 3 + 2;
     if (smem > kFlowSmem) throw InvalidArgument("scheduled solve: system too large");
-    ensure_smem_attr((const void*)k_flow_build<T, double, true>, (int)kFlowSmem);
-    ensure_smem_attr((const void*)k_flow_build<T, double, false>, (int)kFlowSmem);
-    ensure_smem_attr((const void*)k_flow_build<T, float, false>, (int)kFlowSmem);
+    ensure_smem_attr((const void*)k_flow_build<T, true>, (int)kFlowSmem);
+    ensure_smem_attr((const void*)k_flow_build<T, false>, (int)kFlowSmem);
     const int rn = std::max(1, r * n);
     int* d = static_cast<int*>(dev_alloc(sizeof(int) * (B + 2) + rn));
     try {
@@ -356,42 +370,47 @@ static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
         if (r) k_flow_union<T><<<ceil_div(r * n, 64), 64, 0, st>>>(in.vt, B, r * n, mask);
         CNG_LAUNCH("k_flow_union");
         FlowOut o{};
-        k_flow_build<T, double, true><<<B, 32, smem, st>>>(in, d, stat, o);
-        CNG_LAUNCH("k_flow_build");
         std::vector<int> h(B + 2);
-        CNG_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(int) * (B + 2), cudaMemcpyDeviceToHost, st));
-        CNG_CUDA(cudaStreamSynchronize(st));
-        auto refuse = [&](const int* x) {
-            if (x[0]) throw InvalidArgument("scheduled solve: the factors are not real up to powers of i");
-            if (x[1]) throw InvalidArgument("scheduled solve: too many operations per column");
+        auto outcome = [&] {
+            CNG_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(int) * (B + 2), cudaMemcpyDeviceToHost, st));
+            CNG_CUDA(cudaStreamSynchronize(st));
+            if (h[B]) throw InvalidArgument("scheduled solve: the factors are not real up to powers of i");
+            if (h[B + 1]) throw InvalidArgument("scheduled solve: too many operations per column");
+            for (int k = 0; k < B; ++k) h[k] = ceil_div(h[k], kSlots);
         };
-        refuse(h.data() + B);
-        for (int k = 0; k < B; ++k) {
-            h[k] = ceil_div(h[k], kSlots);
-            f->chunks = std::max(f->chunks, h[k]);
+        const int chunk = flow_chunk(f->ncr, 8), per = kSlots * ops;
+        f->chunks = ceil_div(cap, kSlots);
+        if ((size_t)B * f->chunks * chunk > kFlowLoose) {
+            k_flow_build<T, true><<<B, 32, smem, st>>>(in, d, stat, o);
+            CNG_LAUNCH("k_flow_build");
+            outcome();
+            f->chunks = *std::max_element(h.begin(), h.begin() + B);
         }
-        f->nchunk = static_cast<int*>(dev_alloc(sizeof(int) * B));
-        CNG_CUDA(cudaMemcpyAsync(f->nchunk, h.data(), sizeof(int) * B, cudaMemcpyHostToDevice, st));
         f->row = o.row = static_cast<unsigned short*>(dev_alloc(2 * (size_t)B * n));
         f->flags = static_cast<unsigned char*>(dev_alloc(2 * (size_t)n));
         k_flow_flags<<<ceil_div(n, 128), 128, 0, st>>>(n, s.perm, s.rowp, s.colp, s.flip_r, s.flip_c, f->flags);
         CNG_LAUNCH("k_flow_flags");
-        for (int v = 0; v < (s.fp32 ? 2 : 1); ++v) {
-            const int elem = v ? 4 : 8, chunk = flow_chunk(f->ncr, elem);
-            f->sb[v] = o.sb = (size_t)f->chunks * chunk;
-            f->data[v] = o.data = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * o.sb, 16)));
-            const size_t words = (size_t)B * o.sb / 4;
-            if (words)
-                k_flow_clear<<<(int)std::min<size_t>((words + 255) / 256, 152 * 32), 256, 0, st>>>(
-                    o.data, o.sb, B, f->chunks, chunk, kSlots * ops * elem, (unsigned)(f->rows - 1) * 0x10001u);
-            CNG_LAUNCH("k_flow_clear");
-            if (v) k_flow_build<T, float, false><<<B, 32, smem, st>>>(in, d, stat, o);
-            else k_flow_build<T, double, false><<<B, 32, smem, st>>>(in, d, stat, o);
-            CNG_LAUNCH("k_flow_build");
+        auto blocks = [](size_t items) { return (int)std::min<size_t>((items + 255) / 256, 152 * 32); };
+        f->sb[0] = o.sb = (size_t)f->chunks * chunk;
+        f->data[0] = o.data = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * o.sb, 16)));
+        const size_t words = (size_t)B * o.sb / 4;
+        if (words)
+            k_flow_clear<<<blocks(words), 256, 0, st>>>(o.data, o.sb, B, f->chunks, chunk, per * 8,
+                                                        (unsigned)(f->rows - 1) * 0x10001u);
+        CNG_LAUNCH("k_flow_clear");
+        k_flow_build<T, false><<<B, 32, smem, st>>>(in, d, stat, o);
+        CNG_LAUNCH("k_flow_build");
+        if (s.fp32) {
+            f->sb[1] = (size_t)f->chunks * flow_chunk(f->ncr, 4);
+            f->data[1] = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * f->sb[1], 16)));
+            const long long total = (long long)B * f->chunks * per;
+            if (total) k_flow_demote<<<blocks((size_t)total), 256, 0, st>>>(f->data[0], f->data[1], total, per);
+            CNG_LAUNCH("k_flow_demote");
         }
-        CNG_CUDA(cudaMemcpyAsync(h.data(), stat, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+        outcome();
+        f->nchunk = static_cast<int*>(dev_alloc(sizeof(int) * B));
+        CNG_CUDA(cudaMemcpyAsync(f->nchunk, h.data(), sizeof(int) * B, cudaMemcpyHostToDevice, st));
         CNG_CUDA(cudaStreamSynchronize(st));
-        refuse(h.data());
     } catch (...) {
         dev_free(d);
         throw;
