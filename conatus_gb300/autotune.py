@@ -1,4 +1,4 @@
-"""Autotuner of the batched banded solve: the schedule of the step's solve is picked by timing.
+"""Schedules of the batched banded solve: the scheduled solve where it applies, else picked by timing.
 
 Candidates: the band kernel (one warp per system over the LU band, ``cng_banded_set_schedule(h,
 -1)``) and the compact-stream schedules of ``cng_banded_schedules`` (two systems per warp over the
@@ -8,6 +8,7 @@ system per warp with the lanes split over entries and components for small batch
 by time slots fixed at the factorization, a warp per system; and the partitioned solve of small FP64 batches, one
 block of warps per system sweeping its blocks of 32 columns at once). The partitioned solve is a candidate only where the DeviceProblem opts into it (``dev.partitioned``,
 or CONATUS_GB300_PARTITIONED=1): its residuals run up to about 15x those of the sequential sweeps.
+A problem whose systems take the scheduled solve gets it without timing (``choose_solve``).
 Candidates a factor set cannot take (a shared pair, the FP32 form, a batch too large for the
 partitioned solve's responses) are refused by the library and skipped. Each candidate solves
 the step's systems (all buckets, one batched call, the FP32 form with its refinement residual) a
@@ -30,8 +31,8 @@ import os
 
 from ._lib import call
 
-__all__ = ["schedules", "split_schedules", "scheduled_schedules", "partitioned_schedules", "windowed_schedules", "tune_solve", "tune_rhs",
-           "cache"]
+__all__ = ["schedules", "split_schedules", "scheduled_schedules", "partitioned_schedules", "windowed_schedules", "choose_solve",
+           "tune_solve", "tune_rhs", "cache"]
 
 _CACHE: dict = {}
 
@@ -96,6 +97,29 @@ def apply(fs, sched: int) -> None:
             continue
         call("cng_banded_set_schedule", h.h, int(sched))
         h.schedule = int(sched)
+
+
+def choose_solve(dev, key, fs, stream=None) -> dict:
+    """The schedule of a new factor set: the scheduled solve where the systems take it, else the fastest of
+    the others (``tune_solve``). Returns {schedule: ms per solve, or None where nothing was timed}.
+
+    The scheduled solve was the fastest candidate on every configuration: RB 256x64 0.036 ms against 0.161
+    for the next, channel 192x129x192 0.65 against 2.46 (FP32 form 1.33 against 2.11), Burgers 0.013
+    against 0.068, the RB ensembles 1.6x. Timing the others as well took 222 ms of a
+    new problem's first factorization there (16 candidates, four solves each), and ties between schedules
+    19 and 20 changed the bits from run to run."""
+    sig = _signature(dev, fs)
+    if os.environ.get("CONATUS_GB300_SOLVE_SCHEDULE") is None and sig not in _CACHE:
+        like32, like16 = scheduled_schedules()
+        # one system without a Fourier direction: its tau matrix hands each rounding on some 1e5 times
+        # larger, so its border sums keep the order of the split-lane schedules
+        sched = like32 if getattr(dev, "d", 1) == 0 else like16
+        try:
+            apply(fs, sched)
+            return {sched: None}
+        except ValueError:
+            pass                          # not real up to powers of i, or too many operations
+    return tune_solve(dev, key, fs, stream)
 
 
 def tune_solve(dev, key, fs, stream=None, reps: int = 3, candidates=None) -> dict:

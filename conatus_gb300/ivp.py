@@ -104,7 +104,7 @@ class DeviceProblem:
         torch = _torch()
         _lib.lib()
         self.factor_sets = factor_sets      # None: keep every (a, b) factorization, else at most this many
-        self.autotune = True                # time the solve schedules on each new factor set
+        self.autotune = True                # choose the solve schedule of each new factor set
         # let the tuner pick the partitioned solve of small FP64 batches (blocks of 32 columns swept
         # at once): faster on small batches, but its residuals run up to about 15x those of the
         # sequential sweeps (the blocks' separate responses cancel), so it is opted into
@@ -430,8 +430,8 @@ class DeviceProblem:
             self._groups = None
             self._factors[key] = f
             if self.compact and self.autotune:
-                from .autotune import tune_solve
-                self.tuning = tune_solve(self, key, f, stream)
+                from .autotune import choose_solve
+                self.tuning = choose_solve(self, key, f, stream)
         return f
 
     def reset_operators(self) -> None:
