@@ -187,42 +187,15 @@ def solve_kernel(sched: int) -> str:
 # write; it reads the 9 z-groups, 32 modes x 19200 columns, and writes the 12 factor fields, 96
 # points x 19200 columns) and the algorithmic bytes of that launch; the full launch's traffic is
 # taken in the same proportion to its algorithmic bytes (the transform streams its fields once)
-RFFT_TRAFFIC = ((95.617024 + 126.273024) * 1e6, 9 * 19200 * 32 * 16 + 12 * 19200 * 96 * 8,
-                "profiles/k_rfft_axis_channel64x129x64_fp64.md")
-FP64_NOMINAL_TFLOPS = 1.25     # GB300 FP64 (2 DFMA per clock per SM): nominal
-
-
-def fp64_peak(stream, reps=3):
-    """FP64 rate measured here: the library's DFMA loop (cng_dfma_probe, 8 independent chains per
-    thread on every SM), best of ``reps`` CUDA-event timings, TFLOP/s (a fused multiply-add is two
-    flops)."""
-    import ctypes
-    import torch
-    from conatus_gb300._lib import call
-    sink = torch.zeros(1, dtype=torch.float64, device="cuda")
-    fl = ctypes.c_double()
-    sh = stream.cuda_stream
-    call("cng_dfma_probe", 2000, 8, sink.data_ptr(), ctypes.byref(fl), sh)      # warm-up
-    best = None
-    for _ in range(reps):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(stream)
-        call("cng_dfma_probe", 20000, 8, sink.data_ptr(), ctypes.byref(fl), sh)
-        e1.record(stream)
-        e1.synchronize()
-        t = fl.value / (e0.elapsed_time(e1) / 1e3) / 1e12
-        best = t if best is None else max(best, t)
-    return best
+RFFT_TRAFFIC = ((99.117824 + 129.987584) * 1e6, 9 * 19200 * 32 * 16 + 12 * 19200 * 96 * 8,
+                "profiles/k_fx_axis_channel64x129x64_fp64.md")
 
 
 def rfft_roofline(dev, stream, hbm_peak, peak_kind, reps=5):
     """Roofline of the FP64 step's dominant kernel: the x backward real transform of every factor
-    field (k_rfft_axis<double>), launched alone through cng_rfft_axis with the step's shapes.
-    Algorithmic bytes: K complex modes read and L reals written per column and field. FLOPs: the
-    conventional 2.5 L log2 L per real transform of length L. The kernel is bound by the FP64 pipe
-    (GB300 issues FP64 at 1/64 of the FP32 rate), so its HBM fraction is low by construction; the
-    FP64 fraction is against the FP64 rate measured in the same run (cng_dfma_probe)."""
-    import math
+    field (k_fx_axis, 64-bit fixed point), launched alone through cng_rfft_axis with the step's
+    shapes. Algorithmic bytes: K complex modes read and L reals written per column and field. The
+    integer products and additions and shared memory bound it, not HBM."""
     import torch
     from conatus_gb300._lib import call
     g = dev.grid
@@ -245,25 +218,17 @@ def rfft_roofline(dev, stream, hbm_peak, peak_kind, reps=5):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / reps
     nbytes = nf * inner * (16 * K + 8 * L)
-    flops = nf * inner * 2.5 * L * math.log2(L)
     achieved = nbytes / (ms / 1e3) / 1e9
     small_traffic, small_bytes, src = RFFT_TRAFFIC
     traffic = small_traffic * nbytes / small_bytes if small_traffic else None
     del x, y
-    peak64 = fp64_peak(stream)
-    return {"kernel": f"k_rfft_axis<double> (x backward, {nf} factor fields, {K} modes -> {L} points, "
+    return {"kernel": f"k_fx_axis<true, false> (x backward, {nf} factor fields, {K} modes -> {L} points, "
                       f"{inner} columns), launched alone",
             "bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
             "traffic": traffic,
             "traffic_source": (src + " (traffic / algorithmic bytes of the F pipeline's launch, small case)")
             if traffic else None,
-            "algorithmic_bytes": nbytes, "launch_ms": ms, "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
-            "binding_roof": {"pipe": "fp64", "achieved_tflops": flops / (ms / 1e3) / 1e12,
-                             "peak_tflops": peak64,
-                             "peak_kind": "measured (cng_dfma_probe: FP64 fused multiply-add loop, this run)",
-                             "nominal_tflops": FP64_NOMINAL_TFLOPS,
-                             "frac": flops / (ms / 1e3) / 1e12 / peak64,
-                             "flops": flops, "flop_count": "2.5 L log2 L per real transform"}}
+            "algorithmic_bytes": nbytes, "launch_ms": ms, "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"}
 
 
 def max_over_ranks(x: float) -> float:
@@ -382,7 +347,7 @@ def run_gpu(args):
             "algorithmic_bytes": sb, "launch_ms": solve_ms, "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
             "F_ms": f_ms}
     # the dominant kernel: the batched solve (two launches per step in the FP32 form), unless the
-    # x backward real transform takes longer (the FP64 channel: FP64-pipe bound)
+    # x backward real transform takes longer (the FP64 channel)
     roof = solve_roof
     if args.precision == "fp64" and dev.d >= 1:
         rf = rfft_roofline(dev, s, hbm_peak, peak_kind)
@@ -564,15 +529,13 @@ def form_fp32(P, C0, cfg, args):
 
 
 def _schedule_summary(dev):
-    """The solve schedule the autotuner kept (-1: band kernel; k >= 0: compact schedule k) and the
-    time per solve it measured for each candidate."""
-    from conatus_gb300 import autotune
-    cache = autotune.cache()
+    """The solve schedule of the problem's factors (-1: band kernel; k >= 0: compact schedule k) and the
+    time per solve of each candidate, where candidates were timed."""
     for fs in reversed(list(dev._factors.values())):          # the problem's own factor sets
-        hit = cache.get(autotune._signature(dev, fs))
-        if hit:
-            best, times = hit
-            return {"chosen": best, "ms_per_solve": {str(k): round(v, 4) for k, v in times.items()}}
+        for h in fs:
+            if h.h is not None:
+                return {"chosen": getattr(h, "schedule", 0),
+                        "ms_per_solve": {str(k): round(v, 4) for k, v in (dev.tuning or {}).items() if v is not None}}
     return None
 
 
