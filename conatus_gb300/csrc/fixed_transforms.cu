@@ -44,6 +44,7 @@ struct FxAxisArgs {
     FxPlan plan;
     FxC scale;                                   // forward: 1/L (real: 1/2L) times 2^shift, in [1/2, 1)
     int shift;
+    int wide;                                    // real backward: every pair of the output is 16-byte aligned
     Expand<double> ex;
 };
 
@@ -248,11 +249,11 @@ __device__ __forceinline__ void fx_axis_body(unsigned bid, const FxAxisArgs& a) 
             } else if constexpr (REAL) {
                 double* d = static_cast<double*>(a.out) + (o * L + k) * (long long)a.inner + 2 * col;
                 const double x = fc.to(v.y, 0), y = fc.to(v.x, 0);
-                if (a.inner & 1) {
+                if (a.wide) {
+                    *reinterpret_cast<double2*>(d) = make_double2(x, y);
+                } else {
                     d[0] = x;
                     if (pair) d[1] = y;
-                } else {
-                    *reinterpret_cast<double2*>(d) = make_double2(x, y);
                 }
             } else {
                 static_cast<double2*>(a.out)[(o * L + k) * (long long)a.inner + col] =
@@ -574,7 +575,9 @@ void fx_axis(const std::vector<FxAxisJob>& jobs, bool real, bool forward, cudaSt
         const FxDeviceTables& t = fx_device_tables(j.L);
         const long long cols = real ? (j.inner + 1) / 2 : j.inner;
         const int lc = fx_log_cols(j.L, cols * j.outer, j.maxseq, false);
-        FxAxisArgs a{j.in, j.out, j.outer, j.inner, std::max(j.ncompact, 0), lc, t.plan, FxC{}, 0, j.ex};
+        // a caller's reals may start 8 bytes off (a slice of a buffer)
+        const int wide = j.inner % 2 == 0 && reinterpret_cast<uintptr_t>(j.out) % 16 == 0;
+        FxAxisArgs a{j.in, j.out, j.outer, j.inner, std::max(j.ncompact, 0), lc, t.plan, FxC{}, 0, wide, j.ex};
         a.scale = fx_scale(1.0L / ((real ? 2.0L : 1.0L) * j.L), a.shift);
         args.push_back(a);
         blocks.push_back(fx_blocks(j.outer * ((cols + (1 << lc) - 1) >> lc)));
