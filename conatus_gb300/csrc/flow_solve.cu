@@ -178,6 +178,9 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
     for (int i = lane; i < n; i += 32) {
         ord[i] = name[i];                        // from here on the name of the row at a position
         if constexpr (!COUNT) o.row[(size_t)sys * n + i] = name[i];
+        // the solve applies the batch's phase of row i: this system's has to be the same (the batch's are
+        // found on a sample of the systems)
+        if (rowph[name[i]] != phase_of(p, i)) bad = 1;
     }
     __syncwarp();
     auto dinv_of = [&](int j) { return real_part_of(ab[(size_t)j * ldab + kv], phase_of(q, j) - rowph[j], bad); };
@@ -199,8 +202,9 @@ __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int
         for (int t0 = 0; t0 < min(kl, n - 1 - j); t0 += 32) {
             const int t = t0 + lane;
             if (t0) a = low(j, t);
-            const double v = real_part_of(a, pure_imag(a) ? 1 - 2 * rowph[j] : 0, bad);
-            put(v != 0.0, src, v != 0.0 ? ord[j + 1 + t] : 0, v, false);
+            const int dst = j + 1 + t < n ? ord[j + 1 + t] : src;
+            const double v = real_part_of(a, rowph[dst] - rowph[j], bad);
+            put(v != 0.0, src, v != 0.0 ? dst : 0, v, false);
         }
     }
     ahead = high(n - 1, 1 + lane);

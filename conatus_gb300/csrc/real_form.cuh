@@ -28,8 +28,8 @@ template <class T>
 __device__ __forceinline__ T phase_in(T b, int p) { return p ? T(b.im, flip(b.re)) : b; }
 
 // Row and column phases of the assembled systems (band `ab` and border rows `vt`, before the
-// factorization), found on up to 256 of them; false where there are none. What is built from the
-// factors checks every value against them.
+// factorization), found on every (batch / 256)-th of them; false where there are none. What is built from
+// the factors has to check every value and every row's phase of every system against them.
 bool find_phases(const zd* ab, const zd* vt, int batch, int n, int r, int kv, int ldab, cudaStream_t st,
                  std::vector<unsigned char>& row, std::vector<unsigned char>& col);
 
