@@ -36,7 +36,8 @@
 namespace cng {
 
 static constexpr int kWarpsPerBlock = 4;
-static constexpr size_t kFlowAutoBytes = (size_t)1 << 30;     // most bytes of operations a host-built handle adds
+// most bytes of operations a host-built handle adds, as allocated (whole chunks: at least 6 KB a system)
+static constexpr size_t kFlowAutoBytes = (size_t)1 << 30;
 static constexpr size_t kMaxSolveSmem = 200 * 1024;   // bytes of shared memory for the y vectors
 
 template <class T>
@@ -730,6 +731,7 @@ struct Banded {
     unsigned char* rowp = nullptr;
     unsigned char* colp = nullptr;
     std::unique_ptr<FlowForm> flow;
+    size_t flow_most = 0;           // its limit in bytes where it was built unasked (0: no limit)
     // shared-pattern refactorization data (create_shared)
     int nnz = 0;
     long long* bulk_dest = nullptr;
@@ -868,15 +870,26 @@ static void detect_phases(Banded& h, cudaStream_t st) {
     h.real_form = true;
 }
 
-// the scheduled solve of the factors at hand (refused with InvalidArgument where it does not apply)
+// the scheduled solve of the factors at hand (refused with InvalidArgument where it does not apply, or needs
+// more than flow_most bytes)
 static void build_flow(Banded& h, int lanes, cudaStream_t st) {
     bool in_order = true;
     for (int i = 0; i < h.n; ++i) in_order = in_order && h.perm_host[i] == i;
     const FlowSource s{h.dtype, h.batch, h.n, h.r, h.kl, h.ku, h.ldab, h.ab, h.ipiv, h.vt, h.w, h.slu, h.spiv, h.perm, in_order,
                        h.real_form ? h.rowp : nullptr, h.real_form ? h.colp : nullptr,
-                       h.shared ? h.flip_r : nullptr, h.shared ? h.flip_c : nullptr, h.fp32_ready, lanes};
+                       h.shared ? h.flip_r : nullptr, h.shared ? h.flip_c : nullptr, h.fp32_ready, lanes, h.flow_most};
     h.flow.reset();
     h.flow = flow_build(s, st);
+}
+
+// Operations that nobody asked for: left out where they do not apply or the device has no room for them.
+static void build_flow_unasked(Banded& h, int lanes, cudaStream_t st) {
+    h.flow_most = kFlowAutoBytes;
+    try {
+        build_flow(h, lanes, st);
+    } catch (const InvalidArgument&) {
+    } catch (const DeviceMemoryFull&) {
+    }
 }
 
 static void launch_factor(Banded& h, cudaStream_t st) {
@@ -1105,7 +1118,10 @@ static void make_fp32(Banded& h, cudaStream_t st) {
     if (h.compact_ready) demote_compact(h, st);
     CNG_CUDA(cudaStreamSynchronize(st));
     h.fp32_ready = true;
-    if (h.flow) build_flow(h, h.flow->lanes, st);
+    if (h.flow) {
+        if (h.flow_most) build_flow_unasked(h, h.flow->lanes, st);
+        else build_flow(h, h.flow->lanes, st);
+    }
 }
 
 static void prepare_transpose(Banded& h, cudaStream_t st) {
@@ -1216,14 +1232,10 @@ int cng_banded_create_csr(int dtype, int batch, int n, const int32_t* indptr, co
         CNG_CUDA(cudaEventRecord(ev.e0, st));
         launch_factor(*h, st);
         finish_factor(*h, st, ev.e0, ev.e1);
-        // n = 262 complex, 128 systems: the band kernel takes 570 us. What the form does not take (values
-        // that are not real up to powers of i) and what it would need too much memory for stay with it
-        if ((size_t)h->batch * n * kFlowColumnBytes <= kFlowAutoBytes) {
-            try {
-                build_flow(*h, 32, st);
-            } catch (const InvalidArgument&) {
-            }
-        }
+        // n = 262 complex, 128 systems: 27 us, the band kernel 290. What the form does not take (values that
+        // are not real up to powers of i) and what it would need too much memory for stay with that
+        // kernel; batches that are too large by their columns alone are not counted first
+        if ((size_t)h->batch * n * kFlowColumnBytes <= kFlowAutoBytes) build_flow_unasked(*h, 32, st);
         *out = reinterpret_cast<cng_banded*>(h.release());
     })
 }
@@ -3434,6 +3446,7 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
             const int lanes = sched == cng::kFlow32 ? 32 : 16;       // of a border sum
             if (lanes == 32 && h->shared)
                 throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
+            h->flow_most = 0;                      // asked for
             if (!h->flow || h->flow->lanes != lanes) cng::build_flow(*h, lanes, nullptr);
         } else {
             h->flow.reset();                       // another schedule: the operations are not kept

@@ -34,6 +34,9 @@ struct RuntimeFailure : std::runtime_error {
 struct CudaFailure : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
+struct DeviceMemoryFull : CudaFailure {      // the same status; optional memory can be done without
+    using CudaFailure::CudaFailure;
+};
 
 void set_error(const std::string& msg);
 

@@ -390,6 +390,8 @@ static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
             outcome();
             f->chunks = *std::max_element(h.begin(), h.begin() + B);
         }
+        const size_t each = (size_t)f->chunks * (chunk + (s.fp32 ? flow_chunk(f->ncr, 4) : 0)) + 2 * (size_t)n + sizeof(int);
+        if (s.most && each * B > s.most) throw InvalidArgument("scheduled solve: too much memory");
         f->row = o.row = static_cast<unsigned short*>(dev_alloc(2 * (size_t)B * n));
         f->flags = static_cast<unsigned char*>(dev_alloc(2 * (size_t)n));
         k_flow_flags<<<ceil_div(n, 128), 128, 0, st>>>(n, s.perm, s.rowp, s.colp, s.flip_r, s.flip_c, f->flags);

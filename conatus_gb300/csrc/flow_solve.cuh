@@ -28,6 +28,7 @@ struct FlowSource {                      // the factored handle's arrays (banded
     const unsigned char* flip_c;
     bool fp32;                           // also the FP32 copies (mixed form)
     int lanes;                           // lanes of a border sum: 16 or 32
+    size_t most;                         // most bytes of operations (0: what the device has)
 };
 
 struct FlowForm {
@@ -48,7 +49,7 @@ struct FlowForm {
 };
 
 // Throws InvalidArgument where the form does not apply (size, fill, or values that are not real up to
-// the phases). Waits for `st`.
+// the phases) or takes more than `most` bytes. Waits for `st`.
 std::unique_ptr<FlowForm> flow_build(const FlowSource& s, cudaStream_t st);
 
 struct FlowJob {

@@ -31,8 +31,9 @@ void* dev_alloc(size_t bytes) {
     const cudaError_t e = cudaMalloc(&q, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        throw CudaFailure(std::string("cudaMalloc of ") + std::to_string(bytes) + " bytes failed: " +
-                          cudaGetErrorString(e));
+        const std::string what = std::string("cudaMalloc of ") + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e);
+        if (e == cudaErrorMemoryAllocation) throw DeviceMemoryFull(what);
+        throw CudaFailure(what);
     }
     Pool& p = pool();
     try {

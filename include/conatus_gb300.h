@@ -166,7 +166,7 @@ int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_
  * operations (allocates, runs on the legacy default stream and waits for it; freed when another
  * schedule is set) and refuses (status 1) systems that are not real up to powers of i and more than
  * 400 bytes of operations per column. Handles of cng_banded_create_csr hold them from the start where
- * they apply (up to 1 GB), in place of the band kernel's solve.
+ * they apply and take at most 1 GB of free memory, in place of the band kernel's solve.
  * Setting the partitioned schedule builds its responses to unit window values (allocates, runs on
  * the legacy default stream and waits for it) and refuses (status 1) shared pairs, kl > 16,
  * kl + ku > 32, n > 1024 and responses above 256 MB; its solves refuse the FP32 factors and
