@@ -30,6 +30,7 @@ import functools
 import os
 
 from ._lib import call
+from .errors import DeviceMemoryError
 
 __all__ = ["schedules", "split_schedules", "scheduled_schedules", "partitioned_schedules", "windowed_schedules", "choose_solve",
            "tune_solve", "tune_rhs", "cache"]
@@ -117,8 +118,8 @@ def choose_solve(dev, key, fs, stream=None) -> dict:
         try:
             apply(fs, sched)
             return {sched: None}
-        except ValueError:
-            pass                          # not real up to powers of i, or too many operations
+        except (ValueError, DeviceMemoryError):
+            pass                          # not real up to powers of i, too many operations, or no room
     return tune_solve(dev, key, fs, stream)
 
 
@@ -167,9 +168,9 @@ def tune_solve(dev, key, fs, stream=None, reps: int = 3, candidates=None) -> dic
             e1.record(st)
             e1.synchronize()
             times[sched] = e0.elapsed_time(e1) / reps
-        except ValueError:
-            continue                      # schedule does not fit (shared memory), or does not solve
-                                          # shared pairs: not a candidate
+        except (ValueError, DeviceMemoryError):
+            continue                      # schedule does not fit (shared memory, device memory), or does
+                                          # not solve shared pairs: not a candidate
     if not times:
         raise ValueError("no solve schedule fits these systems (shared memory)")
     best = min(times, key=times.get)

@@ -11,6 +11,10 @@ class CudaError(RuntimeError):
     """A CUDA failure, or the CUDA library is missing (never a silent CPU fallback)."""
 
 
+class DeviceMemoryError(CudaError):
+    """A device allocation failed: what is optional is done without."""
+
+
 class NumericalError(RuntimeError):
     """A run has blown up: its state holds a NaN or an infinity (the reference's
     ``conatus.errors.NumericalError`` of the finite-state check, python/conatus/timestep/
@@ -23,7 +27,8 @@ def check_status(status: int, message: str, where: str) -> None:
     if status == 2:
         raise RuntimeError(message)
     if status == 3:
-        raise CudaError(f"{where}: {message}")
+        kind = DeviceMemoryError if message.startswith("cudaMalloc of") and message.endswith("out of memory") else CudaError
+        raise kind(f"{where}: {message}")
     if status == 4:
         raise MemoryError(f"{where}: {message}")
     raise RuntimeError(f"{where}: status {status}: {message}")
