@@ -872,14 +872,19 @@ static void detect_phases(Banded& h, cudaStream_t st) {
 
 // the scheduled solve of the factors at hand (refused with InvalidArgument where it does not apply, or needs
 // more than flow_most bytes)
-static void build_flow(Banded& h, int lanes, cudaStream_t st) {
+static std::unique_ptr<FlowForm> make_flow(const Banded& h, int lanes, cudaStream_t st) {
     bool in_order = true;
     for (int i = 0; i < h.n; ++i) in_order = in_order && h.perm_host[i] == i;
     const FlowSource s{h.dtype, h.batch, h.n, h.r, h.kl, h.ku, h.ldab, h.ab, h.ipiv, h.vt, h.w, h.slu, h.spiv, h.perm, in_order,
                        h.real_form ? h.rowp : nullptr, h.real_form ? h.colp : nullptr,
                        h.shared ? h.flip_r : nullptr, h.shared ? h.flip_c : nullptr, h.fp32_ready, lanes, h.flow_most};
+    return flow_build(s, st);
+}
+
+// in place of those of earlier factors
+static void build_flow(Banded& h, int lanes, cudaStream_t st) {
     h.flow.reset();
-    h.flow = flow_build(s, st);
+    h.flow = make_flow(h, lanes, st);
 }
 
 // Operations that nobody asked for: left out where they do not apply or the device has no room for them.
@@ -3442,24 +3447,19 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
         if (!h) throw InvalidArgument("null handle");
         if (sched < -1 || sched >= kNumSchedules) throw InvalidArgument("schedule out of range");
         if (sched >= 0 && !h->compact_ready) throw InvalidArgument("compact schedules need cng_banded_compact first");
-        if (sched == cng::kFlow32 || sched == cng::kFlow16) {
+        // what the schedule needs first (refused where it does not apply): until it is there, the handle
+        // keeps what it has
+        const bool timed = sched == cng::kFlow32 || sched == cng::kFlow16;
+        std::unique_ptr<cng::FlowForm> flow;
+        if (timed) {
             const int lanes = sched == cng::kFlow32 ? 32 : 16;       // of a border sum
             if (lanes == 32 && h->shared)
                 throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
-            h->flow_most = 0;                      // asked for
-            if (!h->flow || h->flow->lanes != lanes) cng::build_flow(*h, lanes, nullptr);
-        } else {
-            h->flow.reset();                       // another schedule: the operations are not kept
+            if (!h->flow || h->flow->lanes != lanes) flow = cng::make_flow(*h, lanes, nullptr);
         }
-        if (sched == cng::kPartSchedule) {
-            cng::build_part(*h);                   // the responses (refused where it does not apply)
-        } else if (h->part_ready) {                // another schedule: the responses are not kept
-            dev_free(h->p_Rf);
-            dev_free(h->p_Rb);
-            h->p_Rf = h->p_Rb = nullptr;
-            h->part_ready = false;
-        }
-        if (sched >= 0 && cng::kSchedules[sched].split == cng::kWindowFlag) {
+        if (sched == cng::kPartSchedule) cng::build_part(*h);        // the responses
+        const bool windowed = sched >= 0 && cng::kSchedules[sched].split == cng::kWindowFlag;
+        if (windowed) {
             const size_t need = cng::window_scratch_entries(*h);     // the windowed sweeps' scratch
             if (h->w_cap < need) {
                 dev_free(h->w_scr);
@@ -3468,7 +3468,18 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
                 dalloc(&h->w_scr, need, sizeof(zd));
                 h->w_cap = need;
             }
-        } else if (h->w_scr) {                     // another schedule: the scratch is not kept
+        }
+        // another schedule's operations, responses and scratch are not kept
+        if (flow) h->flow = std::move(flow);
+        if (timed) h->flow_most = 0;               // asked for
+        else h->flow.reset();
+        if (sched != cng::kPartSchedule && h->part_ready) {
+            dev_free(h->p_Rf);
+            dev_free(h->p_Rb);
+            h->p_Rf = h->p_Rb = nullptr;
+            h->part_ready = false;
+        }
+        if (!windowed && h->w_scr) {
             dev_free(h->w_scr);
             h->w_scr = nullptr;
             h->w_cap = 0;

@@ -159,7 +159,8 @@ int cng_banded_solve_batch2(int nh, cng_banded* const* h, const void* const* b, 
 int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_t* split);
 /* Schedule of a handle: 0 .. count-1 a compact schedule (needs cng_banded_compact), -1 the band
  * kernel (one warp per system, no compact streams). cng_banded_solve_batch uses the handles'
- * common schedule (schedule 0 when they differ; the band kernel per bucket when all are -1).
+ * common schedule (schedule 0 when they differ; the band kernel per bucket when all are -1). A
+ * schedule that is refused leaves the handle with the one it has.
  * The last two schedules run the sweeps' operations by time slots fixed at the factorization, a warp
  * per system: the last but one (split = 1) with the results of the split-lane schedules, bit for bit,
  * the last with those of schedule 0, shared pairs and FP32 factors as well. Setting one builds its
