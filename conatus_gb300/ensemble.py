@@ -125,8 +125,14 @@ class FourierEnsemble:
     # ------------------------------------------------------------------ state
     def set_state(self, C_list, t: float = 0.0) -> None:
         """Per member, its N/2 complex mode amplitudes (C_0 real)."""
-        # complex vectors as they come (4096 members: a pass of 20 steps 2.04 -> 1.64 ms)
-        flat = np.concatenate(C_list) if all(type(c) is np.ndarray for c in C_list) else None
+        C_list = list(C_list)
+        # complex vectors as they come (4096 members: a pass of 20 steps 2.04 -> 1.64 ms), the rest one by one
+        flat = None
+        if all(type(c) is np.ndarray for c in C_list):
+            try:
+                flat = np.concatenate(C_list)
+            except (TypeError, ValueError):
+                pass                      # several ranks or kinds
         if flat is None or flat.ndim != 1 or flat.dtype != np.complex128:
             flat = np.concatenate([np.asarray(c, np.complex128).ravel() for c in C_list])
         if flat.size != self.n_total:
