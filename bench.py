@@ -415,8 +415,8 @@ def run_gpu(args):
 def subrecords(args):
     """The other configurations, compact and time-bounded, beside the default line: the serving
     stream (100 requests at 200/s, steps U[1000, 20000]; FP64 and the FP32 form under the 150 GB
-    budget, FP64 under a 1.5 GB budget that binds), RB 256x64 and Burgers in FP64 with and without
-    the partitioned solve, the KS ensemble (4096 members, 500 steps) and the RB ensemble (1024 cases
+    budget, FP64 under a 1.5 GB budget that binds), RB 256x64 and Burgers in FP64 with the
+    default schedule and with the partitioned one, the KS ensemble (4096 members, 500 steps) and the RB ensemble (1024 cases
     of three Nz, 50 steps) in the FP32 form."""
     import copy
     import torch
@@ -455,13 +455,15 @@ def subrecords(args):
 
 
 def partitioned_record(steps=100, warmup=5):
-    """RB 256x64 (SBDF2 and RK443) and Burgers N=128 in FP64, graph-replayed steps with the tuner's
-    sequential-sweep schedules and with the partitioned solve allowed, from the same state: steps/s
+    """RB 256x64 (SBDF2 and RK443) and Burgers N=128 in FP64, graph-replayed steps with the schedule
+    that a problem gets by default and with the partitioned one, from the same state: steps/s
     of each and the relative difference of the two final states (the partitioned solve's rounding).
-    100 steps: RB's configured state grows too fast to stay finite past about 200 steps at dt=1e-4."""
+    The partitioned schedule is fixed: a problem that opts into it has it timed beside the scheduled solve,
+    which is the faster one here. 100 steps: RB's configured state grows too fast to stay finite past about 200 steps at dt=1e-4."""
     import torch
-    from conatus_gb300 import workloads as W
+    from conatus_gb300 import autotune, workloads as W
     from conatus_gb300.ivp import DeviceProblem, IVPSolver
+    fixed = str(min(autotune.partitioned_schedules()))
     out = {}
     for name, config, scheme in (("rayleigh_benard_sbdf2", "rayleigh_benard", None),
                                  ("rayleigh_benard_rk443", "rayleigh_benard", "RK443"),
@@ -472,10 +474,17 @@ def partitioned_record(steps=100, warmup=5):
         rec, X = {}, []
         for part in (False, True):
             dev = DeviceProblem(P, "fp64")
-            dev.partitioned = part
             s = IVPSolver(P, scheme=scheme or cfg["scheme"], dt=cfg["dt"], device_problem=dev)
             s.set_state(C0)
-            s.run_graph(max(warmup, s.ring))
+            before = os.environ.get("CONATUS_GB300_SOLVE_SCHEDULE")
+            try:                                   # the factorizations are made during the first steps
+                if part:
+                    os.environ["CONATUS_GB300_SOLVE_SCHEDULE"] = fixed
+                s.run_graph(max(warmup, s.ring))
+            finally:
+                os.environ.pop("CONATUS_GB300_SOLVE_SCHEDULE", None)
+                if before is not None:
+                    os.environ["CONATUS_GB300_SOLVE_SCHEDULE"] = before
             torch.cuda.synchronize()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(s.stream)
@@ -795,8 +804,8 @@ def main():
                          "Rayleigh-Benard case); the CPU baseline times SBDF schemes only")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--partitioned", action="store_true",
-                    help="FP64: let the solve tuner take the partitioned solve of small batches (faster "
-                         "on RB 256x64 and Burgers; residuals up to about 15x the sequential sweeps')")
+                    help="FP64: time the partitioned solve of small batches beside the other schedules and "
+                         "keep the fastest (residuals up to about 15x the sequential sweeps')")
     ap.add_argument("--no-forms", action="store_true", help="channel FP64: skip the FP32 form's line")
     ap.add_argument("--error-steps", type=int, default=None,
                     help="steps of the FP32 form's error run (default: the configuration's length)")

@@ -8,7 +8,8 @@ system per warp with the lanes split over entries and components for small batch
 by time slots fixed at the factorization, a warp per system; and the partitioned solve of small FP64 batches, one
 block of warps per system sweeping its blocks of 32 columns at once). The partitioned solve is a candidate only where the DeviceProblem opts into it (``dev.partitioned``,
 or CONATUS_GB300_PARTITIONED=1): its residuals run up to about 15x those of the sequential sweeps.
-A problem whose systems take the scheduled solve gets it without timing (``choose_solve``).
+A problem whose systems take the scheduled solve gets it without timing unless it opts in
+(``choose_solve``).
 Candidates a factor set cannot take (a shared pair, the FP32 form, a batch too large for the
 partitioned solve's responses) are refused by the library and skipped. Each candidate solves
 the step's systems (all buckets, one batched call, the FP32 form with its refinement residual) a
@@ -102,7 +103,7 @@ def apply(fs, sched: int) -> None:
 
 def choose_solve(dev, key, fs, stream=None) -> dict:
     """The schedule of a new factor set: the scheduled solve where the systems take it, else the fastest of
-    the others (``tune_solve``). Returns {schedule: ms per solve, or None where nothing was timed}.
+    the others (``tune_solve``; so is every schedule of a problem that opts into the partitioned solve). Returns {schedule: ms per solve, or None where nothing was timed}.
 
     The scheduled solve was the fastest candidate on every configuration: RB 256x64 0.036 ms against 0.161
     for the next, channel 192x129x192 0.65 against 2.46 (FP32 form 1.33 against 2.11), Burgers 0.013
@@ -110,7 +111,9 @@ def choose_solve(dev, key, fs, stream=None) -> dict:
     new problem's first factorization there (16 candidates, four solves each), and ties between schedules
     19 and 20 changed the bits from run to run."""
     sig = _signature(dev, fs)
-    if os.environ.get("CONATUS_GB300_SOLVE_SCHEDULE") is None and sig not in _CACHE:
+    # a problem that opts into the partitioned solve (FP64 only) has it timed beside all the others
+    opted = getattr(dev, "partitioned", False) and dev.precision == "fp64"
+    if os.environ.get("CONATUS_GB300_SOLVE_SCHEDULE") is None and sig not in _CACHE and not opted:
         like32, like16 = scheduled_schedules()
         # one system without a Fourier direction: its tau matrix hands each rounding on some 1e5 times
         # larger, so its border sums keep the order of the split-lane schedules
