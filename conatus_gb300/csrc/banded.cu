@@ -36,6 +36,7 @@
 namespace cng {
 
 static constexpr int kWarpsPerBlock = 4;
+constexpr int kPartSchedule = 11;        // the partitioned solve (kSchedules)
 // most bytes of operations a host-built handle adds, as allocated (whole chunks: at least 6 KB a system)
 static constexpr size_t kFlowAutoBytes = (size_t)1 << 30;
 static constexpr size_t kMaxSolveSmem = 200 * 1024;   // bytes of shared memory for the y vectors
@@ -761,6 +762,17 @@ struct Banded {
         return v;
     }
 
+    // the compact streams, and the partitioned solve's responses made from them
+    void drop_streams() {
+        auto drop = [](auto*& p) {
+            dev_free((void*)p);
+            p = nullptr;
+        };
+        drop(c_offL); drop(c_Lrow); drop(c_Lmask); drop(c_offU); drop(c_Udist); drop(c_offV); drop(c_Vcol);
+        drop(c_L); drop(c_U); drop(c_V); drop(c_piv); drop(c_L32); drop(c_U32); drop(c_V32); drop(p_Rf); drop(p_Rb);
+        compact_ready = part_ready = false;
+    }
+
     size_t solve_smem(size_t elem = 0) const {
         const size_t e = elem ? elem : esz;
         return (size_t)kWarpsPerBlock * (size_t)(n + 64 + 2 * std::max(kl, kl + ku + 1) * kChunk) * e;
@@ -1092,6 +1104,8 @@ static void launch_solve(const Banded& h, int io_kind, const SolveIo& io, cudaSt
 }
 
 static void demote_compact(Banded& h, cudaStream_t st);
+static void compact(Banded& h, cudaStream_t st);
+static void build_part(Banded& h);
 
 // FP32 band-kernel solve (one warp per system) of the mixed form: x (+)= A^{-1} b, complex128 data
 static void launch_mixed_dense(const Banded& h, const void* b, void* x, int accumulate, cudaStream_t st) {
@@ -1103,8 +1117,8 @@ static void launch_mixed_dense(const Banded& h, const void* b, void* x, int accu
     CNG_LAUNCH("k_solve_mixed");
 }
 
-static void make_fp32(Banded& h, cudaStream_t st) {
-    if (h.dtype != 1) throw InvalidArgument("FP32 factors need complex128 factors (complex bucket)");
+// the FP32 copies of the factors (not of the compact streams or the scheduled solve's operations)
+static void demote_factors(Banded& h, cudaStream_t st) {
     const size_t B = h.batch, n = h.n, r = h.r;
     if (!h.ab32) dalloc(&h.ab32, B * n * h.ldab, sizeof(zf));
     if (!h.vt32) dalloc(&h.vt32, B * r * n, sizeof(zf));
@@ -1120,6 +1134,11 @@ static void make_fp32(Banded& h, cudaStream_t st) {
     dem(h.vt, h.vt32, (long long)(B * r * n));
     dem(h.w, h.w32, (long long)(B * r * n));
     dem(h.slu, h.slu32, (long long)(B * r * r));
+}
+
+static void make_fp32(Banded& h, cudaStream_t st) {
+    if (h.dtype != 1) throw InvalidArgument("FP32 factors need complex128 factors (complex bucket)");
+    demote_factors(h, st);
     if (h.compact_ready) demote_compact(h, st);
     CNG_CUDA(cudaStreamSynchronize(st));
     h.fp32_ready = true;
@@ -1449,15 +1468,21 @@ int cng_banded_refactor_shared(cng_banded* hh, const void* values, void* stream)
         launch_factor(*h, st);
         h->transposed_ready = false;
         finish_factor(*h, st, ev.e0, ev.e1);
-        if (h->flow) {
-            try {
-                build_flow(*h, h->flow->lanes, st);
-            } catch (const InvalidArgument&) {   // the new values do not take the form: the band kernel
-                h->flow.reset();
-                h->sched = -1;
-            }
+        // what was made from the old factors
+        if (h->fp32_ready) demote_factors(*h, st);
+        if (h->compact_ready) {
+            h->drop_streams();
+            compact(*h, st);
         }
-        if (h->fp32_ready) make_fp32(*h, st);
+        try {
+            if (h->flow) build_flow(*h, h->flow->lanes, st);
+            if (h->sched == kPartSchedule) build_part(*h);
+        } catch (const InvalidArgument&) {       // the new values do not take the schedule
+            h->sched = h->compact_ready ? 0 : -1;
+        } catch (const DeviceMemoryFull&) {
+            h->sched = h->compact_ready ? 0 : -1;
+        }
+        CNG_CUDA(cudaStreamSynchronize(st));
     })
 }
 
@@ -1501,7 +1526,6 @@ struct CompactSchedule { int chunk, stages, split, lanes = 16; };
 // real form, a warp per system): 19 (split = 1) with the split-lane schedules' results, bit for bit, and
 // like them no shared pairs; 20 with schedule 0's, shared pairs as well.
 constexpr int kNumSchedules = 21;
-constexpr int kPartSchedule = 11;
 constexpr int kFlow32 = 19, kFlow16 = 20;
 constexpr int kWindowFlag = 3;
 constexpr CompactSchedule kSchedules[kNumSchedules] = {{8, 2, 0}, {8, 3, 0}, {4, 3, 0}, {16, 2, 0},
@@ -2837,8 +2861,10 @@ static CompactIdx compact_idx(const Banded& h, int chunk = kCChunk) {
 
 static void compact(Banded& h, cudaStream_t st) {
     if (h.dtype != 1) throw InvalidArgument("the compact solve is built for complex128 buckets");
+    if (h.compact_ready) throw InvalidArgument("compact(): already built");
     const int n = h.n, kv = h.kl + h.ku, r = h.r;
     if (kv > 255 || h.kl > 31) throw InvalidArgument("compact solve: band too wide (kl <= 31, kl + ku <= 255)");
+    h.drop_streams();                                        // of a build that failed
     // 1. union masks over the batch
     std::vector<unsigned char> mab((size_t)n * h.ldab), mvt((size_t)std::max(1, r) * n);
     unsigned char* dm = nullptr;
@@ -2912,11 +2938,6 @@ static void compact(Banded& h, cudaStream_t st) {
         for (int s0 = sb; s0 < se; s0 += kPartCH)
             h.p_maxUc = std::max(h.p_maxUc, offU[std::min(s0 + kPartCH, se)] - offU[s0]);
     }
-    // responses of an earlier factor set are stale
-    dev_free(h.p_Rf);
-    dev_free(h.p_Rb);
-    h.p_Rf = h.p_Rb = nullptr;
-    h.part_ready = false;
     h.cL = (int)Lrow.size();
     h.cU = (int)Udist.size();
     h.cV = (int)Vcol.size();
@@ -2927,18 +2948,13 @@ static void compact(Banded& h, cudaStream_t st) {
         dalloc(d, std::max<size_t>(v.size(), 1), sizeof(E));
         if (!v.empty()) CNG_CUDA(cudaMemcpyAsync(*d, v.data(), sizeof(E) * v.size(), cudaMemcpyHostToDevice, st));
     };
-    if (!h.c_offL) {
-        up(&h.c_offL, offL); up(&h.c_Lrow, Lrow); up(&h.c_Lmask, Lmask); up(&h.c_offU, offU);
-        up(&h.c_Udist, Udist); up(&h.c_offV, offV); up(&h.c_Vcol, Vcol);
-        const size_t G = h.cG, W = h.cWg;
-        dalloc(&h.c_L, W * std::max(h.cL, 1) * G, sizeof(zd));
-        dalloc(&h.c_U, W * std::max(h.cU, 1) * G, sizeof(zd));
-        dalloc(&h.c_V, W * std::max(h.cV, 1) * G, sizeof(zd));
-        dalloc(&h.c_piv, W * n * G, sizeof(int));
-    } else {
-        // refactorization: the pattern of the new factors must fit the stored union
-        throw InvalidArgument("compact(): already built; refactor into a new handle");
-    }
+    up(&h.c_offL, offL); up(&h.c_Lrow, Lrow); up(&h.c_Lmask, Lmask); up(&h.c_offU, offU);
+    up(&h.c_Udist, Udist); up(&h.c_offV, offV); up(&h.c_Vcol, Vcol);
+    const size_t G = h.cG, W = h.cWg;
+    dalloc(&h.c_L, W * std::max(h.cL, 1) * G, sizeof(zd));
+    dalloc(&h.c_U, W * std::max(h.cU, 1) * G, sizeof(zd));
+    dalloc(&h.c_V, W * std::max(h.cV, 1) * G, sizeof(zd));
+    dalloc(&h.c_piv, W * n * G, sizeof(int));
     CNG_CUDA(cudaStreamSynchronize(st));
     // 3. pack
     const int total = h.cWg * h.cG;

@@ -65,7 +65,9 @@ int cng_banded_create_shared(int dtype, int batch, int n, const int32_t* indptr,
                              int nnz, const void* values, const int32_t* border, int r, int pivot,
                              void* stream, cng_banded** out);
 
-/* Refactor a shared-pattern handle with new device values (a new a M + b L of the same pattern).
+/* Refactor a shared-pattern handle with new device values (a new a M + b L of the same pattern): the
+ * FP32 copies, compact streams, responses and operations that the handle has are made again, and a
+ * schedule that the new values do not take gives way to schedule 0 (the band kernel without streams).
  * The reference keeps one factorization per (a, b) key (python/conatus/timestep/system.py:58-82). */
 int cng_banded_refactor_shared(cng_banded* h, const void* values, void* stream);
 
