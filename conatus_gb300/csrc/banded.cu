@@ -2883,10 +2883,10 @@ static void compact(Banded& h, cudaStream_t st) {
         }
         CNG_CUDA(cudaStreamSynchronize(st));
     } catch (...) {
-        cudaFree(dm);
+        dev_free(dm);
         throw;
     }
-    cudaFree(dm);
+    dev_free(dm);
     // 2. index lists
     std::vector<int> offL(n + 1, 0), offU(n + 1, 0), offV(r + 1, 0), Vcol;
     std::vector<unsigned char> Lrow, Udist;
