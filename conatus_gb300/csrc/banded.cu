@@ -686,8 +686,10 @@ struct Banded {
     double factor_ms = 0.0;
     double cond_max = 1.0;
     std::vector<int> perm_host;
-    // compact bucket-union form (built by compact())
+    // compact bucket-union form (built by compact(), at once or when a schedule reads it)
     bool compact_ready = false;
+    bool compact_later = false;
+    bool has_compact() const { return compact_ready || compact_later; }
     int cL = 0, cU = 0, cV = 0, cWg = 0;
     int cMaxLk[4] = {0, 0, 0, 0}, cMaxUk[4] = {0, 0, 0, 0};   // largest stream chunk per chunk size 2, 4, 8, 16
     int cMaxLcol = 0, cMaxUcol = 0;                            // most entries of one column (L, U)
@@ -1474,14 +1476,16 @@ int cng_banded_refactor_shared(cng_banded* hh, const void* values, void* stream)
             h->drop_streams();
             compact(*h, st);
         }
+        const bool streams = h->has_compact();
         try {
             if (h->flow) build_flow(*h, h->flow->lanes, st);
             if (h->sched == kPartSchedule) build_part(*h);
         } catch (const InvalidArgument&) {       // the new values do not take the schedule
-            h->sched = h->compact_ready ? 0 : -1;
+            h->sched = streams ? 0 : -1;
         } catch (const DeviceMemoryFull&) {
-            h->sched = h->compact_ready ? 0 : -1;
+            h->sched = streams ? 0 : -1;
         }
+        if (h->sched == 0 && streams && !h->flow && !h->compact_ready) compact(*h, st);
         CNG_CUDA(cudaStreamSynchronize(st));
     })
 }
@@ -1527,6 +1531,7 @@ struct CompactSchedule { int chunk, stages, split, lanes = 16; };
 // like them no shared pairs; 20 with schedule 0's, shared pairs as well.
 constexpr int kNumSchedules = 21;
 constexpr int kFlow32 = 19, kFlow16 = 20;
+static bool is_timed(int sched) { return sched == kFlow32 || sched == kFlow16; }
 constexpr int kWindowFlag = 3;
 constexpr CompactSchedule kSchedules[kNumSchedules] = {{8, 2, 0}, {8, 3, 0}, {4, 3, 0}, {16, 2, 0},
                                                        {16, 3, 0}, {4, 4, 0}, {2, 4, 0}, {16, 4, 0},
@@ -2859,11 +2864,20 @@ static CompactIdx compact_idx(const Banded& h, int chunk = kCChunk) {
     return ix;
 }
 
-static void compact(Banded& h, cudaStream_t st) {
+static void check_compact(const Banded& h) {
     if (h.dtype != 1) throw InvalidArgument("the compact solve is built for complex128 buckets");
     if (h.compact_ready) throw InvalidArgument("compact(): already built");
+    if (h.kl + h.ku > 255 || h.kl > 31) throw InvalidArgument("compact solve: band too wide (kl <= 31, kl + ku <= 255)");
+}
+
+// The streams of a handle whose streams wait for a schedule that reads them.
+static void need_streams(Banded& h, cudaStream_t st) {
+    if (!h.compact_ready && h.compact_later) compact(h, st);
+}
+
+static void compact(Banded& h, cudaStream_t st) {
+    check_compact(h);
     const int n = h.n, kv = h.kl + h.ku, r = h.r;
-    if (kv > 255 || h.kl > 31) throw InvalidArgument("compact solve: band too wide (kl <= 31, kl + ku <= 255)");
     h.drop_streams();                                        // of a build that failed
     // 1. union masks over the batch
     std::vector<unsigned char> mab((size_t)n * h.ldab), mvt((size_t)std::max(1, r) * n);
@@ -3332,11 +3346,13 @@ int cng_banded_solve_batch2(int nh, cng_banded* const* hh, const void* const* b,
         std::vector<const Banded*> hs;
         std::vector<SolveIo> ios, ios2;
         std::vector<int> rng(2 * nh, -1);
-        bool any_pair = false, any_range = false;
+        bool any_pair = false, any_range = false, timed = true, dense = true;
         for (int k = 0; k < nh; ++k) {
             const Banded* h = reinterpret_cast<const Banded*>(hh[k]);
-            if (!h || !h->compact_ready || h->dtype != 1)
+            if (!h || !h->has_compact() || h->dtype != 1)
                 throw InvalidArgument("batched solve needs complex128 handles in compact form");
+            timed = timed && is_timed(h->sched) && h->sched == reinterpret_cast<const Banded*>(hh[0])->sched;
+            dense = dense && h->sched < 0;
             if (range && !(range[2 * k] == 0 && range[2 * k + 1] == h->batch)) {
                 const int s0 = range[2 * k], s1 = range[2 * k + 1];
                 if (s0 < 0 || s1 <= s0 || s1 > h->batch || s0 % h->cG || (s1 % h->cG && s1 != h->batch))
@@ -3367,8 +3383,6 @@ int cng_banded_solve_batch2(int nh, cng_banded* const* hh, const void* const* b,
             ios2.push_back(io2);
         }
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        bool dense = true;
-        for (const Banded* h : hs) dense = dense && h->sched < 0;
         if (dense) {              // the band kernel, one launch per bucket
             if (any_pair) throw InvalidArgument("the band kernel does not solve shared pairs: a compact schedule");
             if (any_range) throw InvalidArgument("the band kernel solves whole batches (no system range)");
@@ -3379,6 +3393,9 @@ int cng_banded_solve_batch2(int nh, cng_banded* const* hh, const void* const* b,
             }
             return CNG_OK;
         }
+        // schedules that differ fall back on schedule 0: its streams, if they still wait
+        if (!timed)
+            for (int k = 0; k < nh; ++k) need_streams(*reinterpret_cast<Banded*>(hh[k]), st);
         if (fp32) {
             std::vector<CompactData<zf>> cds;
             for (const Banded* h : hs)
@@ -3415,7 +3432,7 @@ int cng_banded_share(cng_banded* hh, const int8_t* dr, const int8_t* dc, void* s
         cng::Banded* h = reinterpret_cast<cng::Banded*>(hh);
         if (!h || !dr || !dc) throw InvalidArgument("null argument");
         if (h->dtype != 1) throw InvalidArgument("shared factors: complex128 handles");
-        if (h->compact_ready) throw InvalidArgument("cng_banded_share must come before cng_banded_compact");
+        if (h->has_compact()) throw InvalidArgument("cng_banded_share must come before cng_banded_compact");
         const int n = h->n;
         std::vector<unsigned char> fr(n), fc(n);
         for (int i = 0; i < n; ++i) {
@@ -3445,6 +3462,16 @@ int cng_banded_compact(cng_banded* hh, void* stream) {
     CNG_TRY({ cng::compact(*reinterpret_cast<cng::Banded*>(hh), static_cast<cudaStream_t>(stream)); })
 }
 
+int cng_banded_compact_later(cng_banded* hh) {
+    CNG_TRY({
+        cng::Banded* h = reinterpret_cast<cng::Banded*>(hh);
+        if (!h) throw InvalidArgument("null handle");
+        cng::check_compact(*h);
+        h->cG = h->shared ? 1 : cng::kGroup;
+        h->compact_later = true;
+    })
+}
+
 int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_t* split) {
     CNG_TRY({
         if (!count) throw InvalidArgument("null argument");
@@ -3462,16 +3489,18 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
         cng::Banded* h = reinterpret_cast<cng::Banded*>(hh);
         if (!h) throw InvalidArgument("null handle");
         if (sched < -1 || sched >= kNumSchedules) throw InvalidArgument("schedule out of range");
-        if (sched >= 0 && !h->compact_ready) throw InvalidArgument("compact schedules need cng_banded_compact first");
+        if (sched >= 0 && !h->has_compact()) throw InvalidArgument("compact schedules need cng_banded_compact first");
         // what the schedule needs first (refused where it does not apply): until it is there, the handle
         // keeps what it has
-        const bool timed = sched == cng::kFlow32 || sched == cng::kFlow16;
+        const bool timed = cng::is_timed(sched);
         std::unique_ptr<cng::FlowForm> flow;
         if (timed) {
             const int lanes = sched == cng::kFlow32 ? 32 : 16;       // of a border sum
             if (lanes == 32 && h->shared)
                 throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
             if (!h->flow || h->flow->lanes != lanes) flow = cng::make_flow(*h, lanes, nullptr);
+        } else if (sched >= 0) {
+            cng::need_streams(*h, nullptr);
         }
         if (sched == cng::kPartSchedule) cng::build_part(*h);        // the responses
         const bool windowed = sched >= 0 && cng::kSchedules[sched].split == cng::kWindowFlag;
@@ -3487,8 +3516,12 @@ int cng_banded_set_schedule(cng_banded* hh, int sched) {
         }
         // another schedule's operations, responses and scratch are not kept
         if (flow) h->flow = std::move(flow);
-        if (timed) h->flow_most = 0;               // asked for
-        else h->flow.reset();
+        if (timed) {
+            h->flow_most = 0;                      // asked for
+            if (h->compact_later) h->drop_streams();
+        } else {
+            h->flow.reset();
+        }
         if (sched != cng::kPartSchedule && h->part_ready) {
             dev_free(h->p_Rf);
             dev_free(h->p_Rb);

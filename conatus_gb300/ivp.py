@@ -423,7 +423,9 @@ class DeviceProblem:
                 if rel is not None:
                     call("cng_banded_share", h.h, np.ascontiguousarray(rel[0], np.int8).ctypes.data,
                          np.ascontiguousarray(rel[1], np.int8).ctypes.data, _stream_handle(stream))
-                if self.compact:
+                if self.compact and self.autotune:
+                    call("cng_banded_compact_later", h.h)       # the schedule chosen below may read no streams
+                elif self.compact:
                     call("cng_banded_compact", h.h, _stream_handle(stream))
                 f.append(h)
             del vals_all

@@ -14,8 +14,8 @@ one by one:
   border blocks V^T and W (r x n each), the capacitance LU (r x r)), its FP32 copies in the FP32
   form, and the compact factor streams (bounded above by the band: at most kl entries of L and
   kl + ku + 1 of U per column, r x n of V) with the windowed schedules' scratch (one complex128
-  vector per system slot) or the scheduled solve's operations (at most 400 bytes per column and system,
-  two thirds of that again for their FP32 copies); one transient copy of a M + b L while factoring;
+  vector per system slot), or in their place the scheduled solve's operations (at most 400 bytes per column
+  and system, two thirds of that again for their FP32 copies); one transient copy of a M + b L while factoring;
 * the F pipeline's work buffers (``cng_rhs_create``: the spectra S and two grid buffers).
 
 A shared pair's partner (the (kx, -kz) systems solved with the (kx, +kz) factors) holds no factors;
@@ -62,14 +62,14 @@ def _factor_bytes(b, nsys, precision, compact, shared=False):
         # two systems per warp group, one for a shared pair's primary
         slots = nsys if shared else int(math.ceil(nsys / 2)) * 2
         per = n * kl + n * (kl + ku + 1) + r * n
-        out += slots * (per * _Z + n * 4) + 6 * (n + 1) * 4 + per * 5
+        streams = slots * (per * _Z + n * 4) + 6 * (n + 1) * 4 + per * 5
         if precision == "fp32":
-            out += slots * per * _C
+            streams += slots * per * _C
         # the windowed schedules' scratch (two vectors per warp group), held when the tuner picks one
-        scratch = (2 * nsys if shared else slots) * n * _Z
-        # or the scheduled solve's operations
+        streams += (2 * nsys if shared else slots) * n * _Z
+        # or the scheduled solve's operations in place of both
         flow = nsys * (400 * (n + 64) * (5 if precision == "fp32" else 3) // 3 + 2 * n + 8) + 4 * n
-        out += max(scratch, flow) + 2 * n
+        out += max(streams, flow) + 2 * n
     return out
 
 

@@ -109,6 +109,9 @@ int cng_banded_solve_transpose(const cng_banded* h, void* b, void* stream);
  * reference's GPU path drops the zeros of the factors per system instead (level-scheduled streams,
  * core/src/cuda/banded.cu:824-1121). */
 int cng_banded_compact(cng_banded* h, void* stream);
+/* The same, but the streams are made when a schedule that reads them is set (or a batched solve falls
+ * back on schedule 0), and freed when the scheduled solve, which reads none, is. */
+int cng_banded_compact_later(cng_banded* h);
 
 /* One launch solving nh (<= 8) compact complex128 handles: x[k] = A_k^{-1} b[k] (fp32: with the FP32
  * factors, accumulate: x += ...). The buckets of a whole step in one launch, large ones first,
