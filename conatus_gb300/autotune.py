@@ -94,10 +94,9 @@ def _signature(dev, fs):
 
 
 def apply(fs, sched: int) -> None:
-    for h in fs:
-        if h.h is None:                   # a shared pair's partner: solved with its primary's schedule
-            continue
-        call("cng_banded_set_schedule", h.h, int(sched))
+    own = [h for h in fs if h.h is not None]     # a shared pair's partner is solved with its primary's schedule
+    call("cng_banded_set_schedule_all", len(own), (ctypes.c_void_p * len(own))(*[h.h.value for h in own]), int(sched))
+    for h in own:
         h.schedule = int(sched)
 
 

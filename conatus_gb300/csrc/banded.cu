@@ -702,7 +702,6 @@ struct Banded {
     // windowed schedules: the scratch the sweeps spill finished rows to ([cWg][kGroup][n], room
     // for complex128; allocated by cng_banded_set_schedule)
     void* w_scr = nullptr;
-    size_t w_cap = 0;               // entries
     int sched = 0;                 // compact solve schedule (index into kSchedules); -1: band kernel
     int cG = 2;                     // systems per warp group of the compact streams (1: shared pair)
     bool shared = false;            // factors shared with a sign-similar partner bucket
@@ -884,21 +883,20 @@ static void detect_phases(Banded& h, cudaStream_t st) {
     h.real_form = true;
 }
 
-// the scheduled solve of the factors at hand (refused with InvalidArgument where it does not apply, or needs
-// more than flow_most bytes)
-static std::unique_ptr<FlowForm> make_flow(const Banded& h, int lanes, cudaStream_t st) {
+// what the scheduled solve is built from
+static FlowSource flow_source(const Banded& h, int lanes) {
     bool in_order = true;
     for (int i = 0; i < h.n; ++i) in_order = in_order && h.perm_host[i] == i;
-    const FlowSource s{h.dtype, h.batch, h.n, h.r, h.kl, h.ku, h.ldab, h.ab, h.ipiv, h.vt, h.w, h.slu, h.spiv, h.perm, in_order,
+    return FlowSource{h.dtype, h.batch, h.n, h.r, h.kl, h.ku, h.ldab, h.ab, h.ipiv, h.vt, h.w, h.slu, h.spiv, h.perm, in_order,
                        h.real_form ? h.rowp : nullptr, h.real_form ? h.colp : nullptr,
                        h.shared ? h.flip_r : nullptr, h.shared ? h.flip_c : nullptr, h.fp32_ready, lanes, h.flow_most};
-    return flow_build(s, st);
 }
 
-// in place of those of earlier factors
+// the scheduled solve of the factors at hand, in place of that of earlier ones (refused with InvalidArgument
+// where it does not apply, or needs more than flow_most bytes)
 static void build_flow(Banded& h, int lanes, cudaStream_t st) {
     h.flow.reset();
-    h.flow = make_flow(h, lanes, st);
+    h.flow = std::move(flow_build({flow_source(h, lanes)}, st)[0]);
 }
 
 // Operations that nobody asked for: left out where they do not apply or the device has no room for them.
@@ -1538,6 +1536,7 @@ constexpr CompactSchedule kSchedules[kNumSchedules] = {{8, 2, 0}, {8, 3, 0}, {4,
                                                        {8, 2, 1}, {16, 2, 1}, {4, 3, 1}, {8, 2, 2},
                                                        {8, 2, 3}, {4, 3, 3}, {16, 2, 3}, {8, 3, 3},
                                                        {8, 2, 3, 8}, {4, 3, 3, 8}, {8, 3, 3, 8}, {16, 3, 1}, {16, 3, 0}};
+static bool is_windowed(int sched) { return sched >= 0 && kSchedules[sched].split == kWindowFlag; }
 constexpr int kChunkSizes[4] = {2, 4, 8, 16};
 __host__ __device__ constexpr int chunk_index(int ch) { return ch == 2 ? 0 : (ch == 4 ? 1 : (ch == 8 ? 2 : 3)); }
 
@@ -3163,7 +3162,7 @@ static void launch_multi_t(const std::vector<const Banded*>& hs, const std::vect
     }();
     if (WIN)
         for (const Banded* h : hs)
-            if (!h->w_scr || h->w_cap < window_scratch_entries(*h))
+            if (!h->w_scr)
                 throw InvalidArgument("windowed solve: the scratch is not allocated (cng_banded_set_schedule "
                                       "after cng_banded_compact)");
     ensure_smem_attr((const void*)kern, 220 * 1024);
@@ -3332,6 +3331,56 @@ static void launch_multi(const std::vector<const Banded*>& hs, const std::vector
     }
 }
 
+// The streams, responses and scratch that the handle's schedule does not use are not kept.
+static void settle(Banded& h) {
+    if (is_timed(h.sched) && h.compact_later) h.drop_streams();
+    if (h.sched != kPartSchedule && h.part_ready) {
+        dev_free(h.p_Rf);
+        dev_free(h.p_Rb);
+        h.p_Rf = h.p_Rb = nullptr;
+        h.part_ready = false;
+    }
+    if (!is_windowed(h.sched) && h.w_scr) {
+        dev_free(h.w_scr);
+        h.w_scr = nullptr;
+    }
+}
+
+// The schedule of several handles. What it needs is made first (refused where it does not apply): until all
+// of that is there, the handles keep what they have.
+static void set_schedule(const std::vector<Banded*>& hs, int sched) {
+    const int lanes = sched == kFlow32 ? 32 : 16;                // of a border sum of the scheduled solve
+    std::vector<FlowSource> sources;
+    std::vector<Banded*> built;
+    try {
+        for (Banded* h : hs) {
+            if (is_timed(sched)) {
+                if (lanes == 32 && h->shared)
+                    throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
+                if (h->flow && h->flow->lanes == lanes) continue;
+                built.push_back(h);
+                sources.push_back(flow_source(*h, lanes));
+                sources.back().most = 0;                         // asked for
+                continue;
+            }
+            if (sched >= 0) need_streams(*h, nullptr);
+            if (sched == kPartSchedule) build_part(*h);          // the responses
+            if (is_windowed(sched) && !h->w_scr) dalloc(&h->w_scr, window_scratch_entries(*h), sizeof(zd));
+        }
+        auto flows = flow_build(sources, nullptr);
+        for (size_t k = 0; k < built.size(); ++k) built[k]->flow = std::move(flows[k]);
+    } catch (...) {
+        for (Banded* h : hs) settle(*h);
+        throw;
+    }
+    for (Banded* h : hs) {
+        if (is_timed(sched)) h->flow_most = 0;
+        else h->flow.reset();
+        h->sched = sched;
+        settle(*h);
+    }
+}
+
 }  // namespace cng
 
 extern "C" {
@@ -3485,55 +3534,21 @@ int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_
 }
 
 int cng_banded_set_schedule(cng_banded* hh, int sched) {
+    return cng_banded_set_schedule_all(1, &hh, sched);
+}
+
+int cng_banded_set_schedule_all(int nh, cng_banded* const* hh, int sched) {
     CNG_TRY({
-        cng::Banded* h = reinterpret_cast<cng::Banded*>(hh);
-        if (!h) throw InvalidArgument("null handle");
-        if (sched < -1 || sched >= kNumSchedules) throw InvalidArgument("schedule out of range");
-        if (sched >= 0 && !h->has_compact()) throw InvalidArgument("compact schedules need cng_banded_compact first");
-        // what the schedule needs first (refused where it does not apply): until it is there, the handle
-        // keeps what it has
-        const bool timed = cng::is_timed(sched);
-        std::unique_ptr<cng::FlowForm> flow;
-        if (timed) {
-            const int lanes = sched == cng::kFlow32 ? 32 : 16;       // of a border sum
-            if (lanes == 32 && h->shared)
-                throw InvalidArgument("this scheduled solve does not solve shared pairs: a compact two-system schedule");
-            if (!h->flow || h->flow->lanes != lanes) flow = cng::make_flow(*h, lanes, nullptr);
-        } else if (sched >= 0) {
-            cng::need_streams(*h, nullptr);
+        if (nh < 1 || !hh) throw InvalidArgument("no handle");
+        std::vector<cng::Banded*> hs;
+        for (int k = 0; k < nh; ++k) {
+            auto* h = reinterpret_cast<cng::Banded*>(hh[k]);
+            if (!h) throw InvalidArgument("null handle");
+            if (sched < -1 || sched >= kNumSchedules) throw InvalidArgument("schedule out of range");
+            if (sched >= 0 && !h->has_compact()) throw InvalidArgument("compact schedules need cng_banded_compact first");
+            hs.push_back(h);
         }
-        if (sched == cng::kPartSchedule) cng::build_part(*h);        // the responses
-        const bool windowed = sched >= 0 && cng::kSchedules[sched].split == cng::kWindowFlag;
-        if (windowed) {
-            const size_t need = cng::window_scratch_entries(*h);     // the windowed sweeps' scratch
-            if (h->w_cap < need) {
-                dev_free(h->w_scr);
-                h->w_scr = nullptr;
-                h->w_cap = 0;
-                dalloc(&h->w_scr, need, sizeof(zd));
-                h->w_cap = need;
-            }
-        }
-        // another schedule's operations, responses and scratch are not kept
-        if (flow) h->flow = std::move(flow);
-        if (timed) {
-            h->flow_most = 0;                      // asked for
-            if (h->compact_later) h->drop_streams();
-        } else {
-            h->flow.reset();
-        }
-        if (sched != cng::kPartSchedule && h->part_ready) {
-            dev_free(h->p_Rf);
-            dev_free(h->p_Rb);
-            h->p_Rf = h->p_Rb = nullptr;
-            h->part_ready = false;
-        }
-        if (!windowed && h->w_scr) {
-            dev_free(h->w_scr);
-            h->w_scr = nullptr;
-            h->w_cap = 0;
-        }
-        h->sched = sched;
+        cng::set_schedule(hs, sched);
     })
 }
 

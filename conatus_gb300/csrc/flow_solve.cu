@@ -25,6 +25,7 @@
 #include "flow_solve.cuh"
 
 #include <algorithm>
+#include <utility>
 
 #include "real_form.cuh"
 
@@ -35,7 +36,7 @@ constexpr int kRing = 3;                         // chunks staged in shared memo
                                                  // 9, channel 128 x 129 x 128 351 us against 298)
 constexpr int kFlowWarps = 4;                    // most systems of a block
 constexpr size_t kFlowSmem = 220 * 1024;
-constexpr size_t kFlowLoose = 64 << 20;           // bytes of operations laid out at their most, uncounted
+constexpr size_t kFlowLoose = 64 << 20;           // bytes of operations laid out at their most and left so
 constexpr int kMaxBorder = 64;
 constexpr unsigned kFresh = 0x80000000u;         // the operation's sum starts from 0
 
@@ -127,10 +128,9 @@ struct FlowPlan {
 
 // One warp per system: its slots into nslot and, unless COUNT, its operations.
 // stat[0]: not of the form, stat[1]: more slots than allowed.
-// What bounds it: the latency of one warp, 1.7 ms for n = 522, whatever the number of systems. So a batch
-// whose operations fit 64 MB at their most is written without the counting pass, and the FP32 copies are
-// rounded from the others (a third pass before): factorization of channel 96 x 129 x 96 61 -> 57 ms, with FP32
-// copies 69 -> 59, of 128 host-built systems of n = 262 12.0 -> 10.5 ms (10.5 without the operations too).
+// What bounds it: the latency of one warp, 1.7 ms for n = 522, whatever the number of systems. So the
+// operations are written without a counting pass, at their most, and packed where that is more than 64 MB; the
+// counting pass is for host-built handles, whose bytes are limited, and where the device has no room.
 template <class T, bool COUNT>
 __global__ void __launch_bounds__(32) k_flow_build(FlowIn<T> in, int* nslot, int* stat, FlowOut o) {
     extern __shared__ __align__(16) unsigned char fsm[];
@@ -312,6 +312,14 @@ __global__ void k_flow_clear(unsigned char* data, size_t sb, int batch, int chun
     }
 }
 
+// a system's first bytes, laid out closer
+__global__ void k_flow_pack(const int4* __restrict__ in, size_t from, int4* __restrict__ out, size_t to, size_t total) {
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const size_t sys = e / to;
+        out[e] = in[sys * from + (e - sys * to)];
+    }
+}
+
 // the FP32 copies: the same rows, the values rounded; `per` operations to a chunk
 __global__ void k_flow_demote(const unsigned char* __restrict__ in, unsigned char* __restrict__ out, long long total, int per) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
@@ -328,10 +336,11 @@ template <class T>
 __global__ void k_flow_union(const T* __restrict__ vt, int batch, int rn, unsigned char* __restrict__ mask) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= rn) return;
-    unsigned char any = 0;
-    for (int k = 0; k < batch && !any; ++k)
-        if (!is_zero(vt[(size_t)k * rn + q])) any = 1;
-    mask[q] = any;
+    for (int k = blockIdx.y; k < batch; k += gridDim.y)
+        if (!is_zero(vt[(size_t)k * rn + q])) {
+            mask[q] = 1;                         // whichever block is first
+            return;
+        }
 }
 
 __global__ void k_flow_flags(int n, const int* perm, const unsigned char* rowp, const unsigned char* colp,
@@ -347,65 +356,128 @@ static size_t flow_smem(int rows, int ncr, int elem) {
     return (size_t)kRing * flow_chunk(ncr, elem) + ((size_t)rows * ncr * elem + 15) / 16 * 16;
 }
 
-template <class T>
-static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
-    auto f = std::make_unique<FlowForm>();
-    const int n = s.n, r = s.r, B = s.batch;
-    f->n = n; f->batch = B; f->dtype = s.dtype; f->lanes = s.lanes;
-    f->ncr = (s.dtype ? 2 : 1) * (s.flip_r ? 2 : 1);
-    f->rows = n + r * s.lanes + r + 1;
-    f->perm = s.in_order ? nullptr : s.perm;
-    if (f->rows > 32000 || flow_smem(f->rows, f->ncr, 8) > kFlowSmem)
-        throw InvalidArgument("scheduled solve: system too large for shared memory");
-    const int ops = flow_ops(f->ncr);
-    const int cap = std::min(65000, kFlowColumnBytes * (n + 64) / (12 * ops) / kSlots * kSlots);
-    const size_t smem = (size_t)f->rows * 8 + (size_t)n * 7 + (size_t)cap * 3 + 2;
-    if (smem > kFlowSmem) throw InvalidArgument("scheduled solve: system too large");
-    ensure_smem_attr((const void*)k_flow_build<T, true>, (int)kFlowSmem);
-    ensure_smem_attr((const void*)k_flow_build<T, false>, (int)kFlowSmem);
-    const int rn = std::max(1, r * n);
-    int* d = static_cast<int*>(dev_alloc(sizeof(int) * (B + 2) + rn));
-    try {
-        int* stat = d + B;
-        unsigned char* mask = reinterpret_cast<unsigned char*>(d + B + 2);
-        const FlowIn<T> in{s, s.kl + s.ku, f->ncr, f->rows, cap, static_cast<const T*>(s.ab), static_cast<const T*>(s.vt),
-                           static_cast<const T*>(s.w), static_cast<const T*>(s.slu), mask};
-        CNG_CUDA(cudaMemsetAsync(d, 0, sizeof(int) * (B + 2) + rn, st));
-        if (r) k_flow_union<T><<<ceil_div(r * n, 64), 64, 0, st>>>(in.vt, B, r * n, mask);
-        CNG_LAUNCH("k_flow_union");
-        FlowOut o{};
-        std::vector<int> h(B + 2);
-        auto outcome = [&] {
-            CNG_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(int) * (B + 2), cudaMemcpyDeviceToHost, st));
-            CNG_CUDA(cudaStreamSynchronize(st));
-            if (h[B]) throw InvalidArgument("scheduled solve: the factors are not real up to powers of i");
-            if (h[B + 1]) throw InvalidArgument("scheduled solve: too many operations per column");
-            for (int k = 0; k < B; ++k) h[k] = ceil_div(h[k], kSlots);
-        };
-        const int chunk = flow_chunk(f->ncr, 8), per = kSlots * ops;
-        f->chunks = ceil_div(cap, kSlots);
-        if ((size_t)B * f->chunks * chunk > kFlowLoose) {
-            k_flow_build<T, true><<<B, 32, smem, st>>>(in, d, stat, o);
+// One handle's build: its kernels are launched and their outcome fetched in separate calls, so that the
+// builds of several handles run side by side (each takes a warp's latency, whatever its systems).
+struct FlowBuild {
+    FlowSource s;
+    cudaStream_t st;
+    std::unique_ptr<FlowForm> f = std::make_unique<FlowForm>();
+    int* d = nullptr;                            // [batch] slots, the two verdicts, the union of V^T's entries
+    int cap = 0, chunk = 0, per = 0;
+    size_t smem = 0;
+    bool large = false, counted = false;
+    unsigned char* loose = nullptr;              // the operations at their most, once they are packed
+    std::vector<int> h;
+
+    FlowBuild(const FlowSource& src, cudaStream_t stream) : s(src), st(stream), h(src.batch + 2) {}
+    FlowBuild(FlowBuild&& o) : s(o.s), st(o.st), f(std::move(o.f)), d(std::exchange(o.d, nullptr)), h(std::move(o.h)) {}
+    ~FlowBuild() {
+        dev_free(d);
+        dev_free(loose);
+    }
+    static int blocks(size_t items) { return (int)std::min<size_t>((items + 255) / 256, 152 * 32); }
+
+    template <bool COUNT>
+    void launch(const FlowOut& o) {
+        auto go = [&](auto zero) {
+            using T = decltype(zero);
+            ensure_smem_attr((const void*)k_flow_build<T, COUNT>, (int)kFlowSmem);
+            const FlowIn<T> in{s, s.kl + s.ku, f->ncr, f->rows, cap, static_cast<const T*>(s.ab), static_cast<const T*>(s.vt),
+                               static_cast<const T*>(s.w), static_cast<const T*>(s.slu),
+                               reinterpret_cast<const unsigned char*>(d + s.batch + 2)};
+            k_flow_build<T, COUNT><<<s.batch, 32, smem, st>>>(in, d, d + s.batch, o);
             CNG_LAUNCH("k_flow_build");
-            outcome();
+        };
+        if (s.dtype) go(zd(0.0));
+        else go(0.0);
+    }
+    void fetch() {
+        CNG_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(int) * h.size(), cudaMemcpyDeviceToHost, st));
+        CNG_CUDA(cudaStreamSynchronize(st));
+        if (h[s.batch]) throw InvalidArgument("scheduled solve: the factors are not real up to powers of i");
+        if (h[s.batch + 1]) throw InvalidArgument("scheduled solve: too many operations per column");
+        for (int k = 0; k < s.batch; ++k) h[k] = ceil_div(h[k], kSlots);
+    }
+    void begin() {
+        const int n = s.n, r = s.r, B = s.batch;
+        if (r > kMaxBorder || n > 32000) throw InvalidArgument("scheduled solve: too many border rows or columns");
+        if (s.dtype && !s.rowp) throw InvalidArgument("scheduled solve: the systems are not real up to powers of i");
+        f->n = n; f->batch = B; f->dtype = s.dtype; f->lanes = s.lanes;
+        f->ncr = (s.dtype ? 2 : 1) * (s.flip_r ? 2 : 1);
+        f->rows = n + r * s.lanes + r + 1;
+        f->perm = s.in_order ? nullptr : s.perm;
+        if (f->rows > 32000 || flow_smem(f->rows, f->ncr, 8) > kFlowSmem)
+            throw InvalidArgument("scheduled solve: system too large for shared memory");
+        const int ops = flow_ops(f->ncr);
+        cap = std::min(65000, kFlowColumnBytes * (n + 64) / (12 * ops) / kSlots * kSlots);
+        smem = (size_t)f->rows * 8 + (size_t)n * 7 + (size_t)cap * 3 + 2;
+        if (smem > kFlowSmem) throw InvalidArgument("scheduled solve: system too large");
+        const int rn = std::max(1, r * n);
+        d = static_cast<int*>(dev_alloc(sizeof(int) * (B + 2) + rn));
+        CNG_CUDA(cudaMemsetAsync(d, 0, sizeof(int) * (B + 2) + rn, st));
+        unsigned char* mask = reinterpret_cast<unsigned char*>(d + B + 2);
+        const dim3 grid(ceil_div(r * n, 64), std::min(B, 64));     // a zero entry is read in every system
+        if (r && s.dtype) k_flow_union<zd><<<grid, 64, 0, st>>>(static_cast<const zd*>(s.vt), B, r * n, mask);
+        else if (r) k_flow_union<double><<<grid, 64, 0, st>>>(static_cast<const double*>(s.vt), B, r * n, mask);
+        CNG_LAUNCH("k_flow_union");
+        chunk = flow_chunk(f->ncr, 8);
+        per = kSlots * ops;
+        f->chunks = ceil_div(cap, kSlots);
+        large = (size_t)B * f->chunks * chunk > kFlowLoose;
+        if (large && !s.most) {                  // at their most, packed below, where there is room
+            try {
+                f->data[0] = static_cast<unsigned char*>(dev_alloc((size_t)B * f->chunks * chunk));
+            } catch (const DeviceMemoryFull&) {
+            }
+        }
+        counted = large && !f->data[0];
+        if (counted) launch<true>(FlowOut{});
+    }
+    void write() {
+        const int n = s.n, B = s.batch;
+        if (counted) {
+            fetch();
             f->chunks = *std::max_element(h.begin(), h.begin() + B);
         }
         const size_t each = (size_t)f->chunks * (chunk + (s.fp32 ? flow_chunk(f->ncr, 4) : 0)) + 2 * (size_t)n + sizeof(int);
         if (s.most && each * B > s.most) throw InvalidArgument("scheduled solve: too much memory");
+        FlowOut o{};
         f->row = o.row = static_cast<unsigned short*>(dev_alloc(2 * (size_t)B * n));
         f->flags = static_cast<unsigned char*>(dev_alloc(2 * (size_t)n));
+        f->nchunk = static_cast<int*>(dev_alloc(sizeof(int) * B));
         k_flow_flags<<<ceil_div(n, 128), 128, 0, st>>>(n, s.perm, s.rowp, s.colp, s.flip_r, s.flip_c, f->flags);
         CNG_LAUNCH("k_flow_flags");
-        auto blocks = [](size_t items) { return (int)std::min<size_t>((items + 255) / 256, 152 * 32); };
         f->sb[0] = o.sb = (size_t)f->chunks * chunk;
-        f->data[0] = o.data = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * o.sb, 16)));
+        if (!f->data[0]) f->data[0] = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * o.sb, 16)));
+        o.data = f->data[0];
         const size_t words = (size_t)B * o.sb / 4;
         if (words)
             k_flow_clear<<<blocks(words), 256, 0, st>>>(o.data, o.sb, B, f->chunks, chunk, per * 8,
                                                         (unsigned)(f->rows - 1) * 0x10001u);
         CNG_LAUNCH("k_flow_clear");
-        k_flow_build<T, false><<<B, 32, smem, st>>>(in, d, stat, o);
-        CNG_LAUNCH("k_flow_build");
+        launch<false>(o);
+    }
+    void pack() {                                // what was written at its most, where that saves half or more
+        const size_t B = (size_t)s.batch;
+        fetch();
+        const int used = *std::max_element(h.begin(), h.begin() + B);
+        if (!large || 2 * used > f->chunks) return;
+        const size_t to = (size_t)used * chunk;
+        loose = std::exchange(f->data[0], nullptr);
+        f->data[0] = static_cast<unsigned char*>(dev_alloc(std::max<size_t>(B * to, 16)));
+        if (used)
+            k_flow_pack<<<blocks(B * to / 16), 256, 0, st>>>(reinterpret_cast<const int4*>(loose), f->sb[0] / 16,
+                                                            reinterpret_cast<int4*>(f->data[0]), to / 16, B * to / 16);
+        CNG_LAUNCH("k_flow_pack");
+        f->sb[0] = to;
+        f->chunks = used;
+    }
+    void finish() {
+        const int B = s.batch;
+        if (loose) {
+            CNG_CUDA(cudaStreamSynchronize(st));
+            dev_free(std::exchange(loose, nullptr));
+        }
         if (s.fp32) {
             f->sb[1] = (size_t)f->chunks * flow_chunk(f->ncr, 4);
             f->data[1] = static_cast<unsigned char*>(dev_alloc(std::max<size_t>((size_t)B * f->sb[1], 16)));
@@ -413,22 +485,58 @@ static std::unique_ptr<FlowForm> build_t(const FlowSource& s, cudaStream_t st) {
             if (total) k_flow_demote<<<blocks((size_t)total), 256, 0, st>>>(f->data[0], f->data[1], total, per);
             CNG_LAUNCH("k_flow_demote");
         }
-        outcome();
-        f->nchunk = static_cast<int*>(dev_alloc(sizeof(int) * B));
         CNG_CUDA(cudaMemcpyAsync(f->nchunk, h.data(), sizeof(int) * B, cudaMemcpyHostToDevice, st));
         CNG_CUDA(cudaStreamSynchronize(st));
-    } catch (...) {
-        dev_free(d);
-        throw;
     }
-    dev_free(d);
-    return f;
-}
+};
 
-std::unique_ptr<FlowForm> flow_build(const FlowSource& s, cudaStream_t st) {
-    if (s.r > kMaxBorder || s.n > 32000) throw InvalidArgument("scheduled solve: too many border rows or columns");
-    if (s.dtype && !s.rowp) throw InvalidArgument("scheduled solve: the systems are not real up to powers of i");
-    return s.dtype ? build_t<zd>(s, st) : build_t<double>(s, st);
+// up to kMost streams beside `main`, ordered after its work
+struct SideStreams {
+    static constexpr int kMost = 7;
+    cudaStream_t side[kMost] = {};
+    int n = 0;
+    SideStreams(int want, cudaStream_t main) {
+        if (want <= 0) return;
+        EventPair ev;
+        CNG_CUDA(cudaEventRecord(ev.e0, main));
+        for (; n < std::min(want, kMost); ++n) {
+            CNG_CUDA(cudaStreamCreateWithFlags(&side[n], cudaStreamNonBlocking));
+            const cudaError_t e = cudaStreamWaitEvent(side[n], ev.e0, 0);
+            if (e != cudaSuccess) {
+                for (int k = 0; k <= n; ++k) cudaStreamDestroy(side[k]);
+                CNG_CUDA(e);
+            }
+        }
+    }
+    ~SideStreams() {
+        for (int k = 0; k < n; ++k) cudaStreamDestroy(side[k]);
+    }
+};
+
+// One warp a system takes 1.7 ms for n = 522, whatever the other handles do, and 3.0 where a handle has more
+// systems than the SMs hold warps: channel 96 x 129 x 96, four handles (2209 systems the largest), 11.7 ms one
+// after another and counted first, 6.5 side by side, 4.4 with the largest written at its most and packed.
+std::vector<std::unique_ptr<FlowForm>> flow_build(const std::vector<FlowSource>& sources, cudaStream_t st) {
+    const SideStreams side((int)sources.size() - 1, st);
+    std::vector<FlowBuild> b;
+    b.reserve(sources.size());
+    for (size_t k = 0; k < sources.size(); ++k) {
+        const int q = (int)(k % (side.n + 1));
+        b.emplace_back(sources[k], q ? side.side[q - 1] : st);
+    }
+    struct Wait {                                // also where a build is refused with others in flight
+        const std::vector<FlowBuild>& b;
+        ~Wait() {
+            for (const auto& x : b) cudaStreamSynchronize(x.st);
+        }
+    } wait{b};
+    for (auto& x : b) x.begin();
+    for (auto& x : b) x.write();
+    for (auto& x : b) x.pack();
+    for (auto& x : b) x.finish();
+    std::vector<std::unique_ptr<FlowForm>> out;
+    for (auto& x : b) out.push_back(std::move(x.f));
+    return out;
 }
 
 // ---- solve ---------------------------------------------------------------------------------------

@@ -49,8 +49,9 @@ struct FlowForm {
 };
 
 // Throws InvalidArgument where the form does not apply (size, fill, or values that are not real up to
-// the phases) or takes more than `most` bytes. Waits for `st`.
-std::unique_ptr<FlowForm> flow_build(const FlowSource& s, cudaStream_t st);
+// the phases) or takes more than `most` bytes. The handles' builds run side by side after `st`'s work, and
+// are waited for.
+std::vector<std::unique_ptr<FlowForm>> flow_build(const std::vector<FlowSource>& sources, cudaStream_t st);
 
 struct FlowJob {
     const FlowForm* form;

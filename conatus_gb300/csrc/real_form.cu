@@ -39,46 +39,47 @@ bool find_phases(const zd* ab, const zd* vt, int batch, int n, int r, int kv, in
         throw;
     }
     dev_free(d);
-    // two-colour rows (nodes 0 .. n-1) and columns (n ..): an entry joins equal (real) or different
-    // (imaginary) phases
-    std::vector<std::vector<std::pair<int, unsigned char>>> adj((size_t)2 * n);
-    auto edge = [&](int i, int j, unsigned char c) {
-        adj[i].push_back({n + j, (unsigned char)(c >> 1)});
-        adj[n + j].push_back({i, (unsigned char)(c >> 1)});
+    // Phases of rows (nodes 0 .. n-1) and columns (n ..): an entry joins equal (real) or different (imaginary)
+    // ones. Sets of joined nodes, each with its phase against the set's root.
+    std::vector<int> up((size_t)2 * n);
+    std::vector<unsigned char> phase((size_t)2 * n, 0);          // against `up`
+    for (int u = 0; u < 2 * n; ++u) up[u] = u;
+    auto root = [&](int u) {
+        unsigned char p = 0;
+        int v = u;
+        for (; up[v] != v; v = up[v]) p ^= phase[v];
+        while (up[u] != v) {                                     // the path shortened
+            const int w = up[u];
+            const unsigned char q = phase[u];
+            up[u] = v;
+            phase[u] = p;
+            p ^= q;
+            u = w;
+        }
+        return v;
+    };
+    auto join = [&](int i, int j, unsigned char c) {
+        const int u = root(i), v = root(n + j);                  // i and n + j now hang on their roots
+        const unsigned char want = (unsigned char)((c >> 1) ^ phase[i] ^ phase[n + j]);
+        if (u == v) return want == 0;
+        up[u] = v;
+        phase[u] = want;
+        return true;
     };
     for (int j = 0; j < n; ++j)
         for (int q = 0; q < ldab; ++q) {
             const unsigned char c = cls[(size_t)j * ldab + q];
             const int i = j + q - kv;
-            if (c == 3) return false;
-            if (c && i >= 0 && i < n) edge(i, j, c);
+            if (c == 3 || (c && i >= 0 && i < n && !join(i, j, c))) return false;
         }
     for (int a = 0; a < r; ++a)
         for (int j = 0; j < n; ++j) {
             const unsigned char c = cls[(size_t)na + (size_t)a * n + j];
-            if (c == 3) return false;
-            if (c) edge(a, j, c);
+            if (c == 3 || (c && !join(a, j, c))) return false;
         }
-    std::vector<signed char> phase((size_t)2 * n, -1);
-    std::vector<int> stack;
-    for (int s = 0; s < 2 * n; ++s) {
-        if (phase[s] >= 0) continue;
-        phase[s] = 0;
-        stack.assign(1, s);
-        while (!stack.empty()) {
-            const int u = stack.back();
-            stack.pop_back();
-            for (const auto& e : adj[u]) {
-                const signed char want = (signed char)(phase[u] ^ e.second);
-                if (phase[e.first] < 0) {
-                    phase[e.first] = want;
-                    stack.push_back(e.first);
-                } else if (phase[e.first] != want) {
-                    return false;
-                }
-            }
-        }
-    }
+    for (int u = 0; u < 2 * n; ++u) root(u);
+    for (int u = 0; u < 2 * n; ++u)
+        if (up[u] == u) phase[u] = 0;
     row.assign(phase.begin(), phase.begin() + n);
     col.assign(phase.begin() + n, phase.end());
     return true;

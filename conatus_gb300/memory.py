@@ -15,7 +15,7 @@ one by one:
   form, and the compact factor streams (bounded above by the band: at most kl entries of L and
   kl + ku + 1 of U per column, r x n of V) with the windowed schedules' scratch (one complex128
   vector per system slot), or in their place the scheduled solve's operations (at most 400 bytes per column
-  and system, two thirds of that again for their FP32 copies); one transient copy of a M + b L while factoring;
+  and system, half of that again while they are packed or two thirds for their FP32 copies); one transient copy of a M + b L while factoring;
 * the F pipeline's work buffers (``cng_rhs_create``: the spectra S and two grid buffers).
 
 A shared pair's partner (the (kx, -kz) systems solved with the (kx, +kz) factors) holds no factors;
@@ -67,8 +67,11 @@ def _factor_bytes(b, nsys, precision, compact, shared=False):
             streams += slots * per * _C
         # the windowed schedules' scratch (two vectors per warp group), held when the tuner picks one
         streams += (2 * nsys if shared else slots) * n * _Z
-        # or the scheduled solve's operations in place of both
-        flow = nsys * (400 * (n + 64) * (5 if precision == "fp32" else 3) // 3 + 2 * n + 8) + 4 * n
+        # or the scheduled solve's operations in place of both: those of a large batch are written at their
+        # most and packed where that saves half or more
+        most = 400 * (n + 64)
+        grown = 10 if precision == "fp32" else 9 if nsys * most > 64 << 20 else 6
+        flow = nsys * (most * grown // 6 + 2 * n + 8) + 4 * n
         out += max(streams, flow) + 2 * n
     return out
 

@@ -181,6 +181,8 @@ int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_
  * allocates its scratch (16 bytes x 2 x n per warp group of systems; freed when another schedule
  * is set): two solves of the same systems of h must then not run at the same time. */
 int cng_banded_set_schedule(cng_banded* h, int sched);
+/* The same for nh handles, all or none of them; what they need is made side by side. */
+int cng_banded_set_schedule_all(int nh, cng_banded* const* h, int sched);
 
 /* Mixed precision: keep FP32 (complex64) copies of the FP64 factors (allocates; refreshed by
  * refactor_shared). No reference counterpart: the FP32 + FP64-refinement form of the solve. */
