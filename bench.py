@@ -112,19 +112,26 @@ def measured_peaks():
 
 
 def solve_bytes(dev, fs):
-    """Algorithmic bytes of one batched solve launch, band-equivalent (as the reference's band
+    """Algorithmic bytes of one batched solve launch: right-hand side in and solution out (2 n complex128
+    per system) and the factors, read once for a shared pair. The scheduled solve reads its operations and
+    the rows' names (2 n); the other kernels are counted band-equivalent (as the reference's band
     kernel reads them): per system the band LU (ldab n), V^T and W (2 r n) and the capacitance LU
-    (r r) in the factor precision, pivots (4 n), right-hand side in and solution out (2 n
-    complex128); a shared pair's partner reads its primary's factors in the same sweep (the
-    reference's SharedFactor), so only its right-hand side and solution count."""
+    (r r) in the factor precision, and pivots (4 n)."""
+    import ctypes
+    from conatus_gb300._lib import call
     ef = 8 if dev.precision == "fp32" else 16
     tot = 0
     for h in fs:
         ns, n, r, ldab = h.batch, h.n, h.rank, h.ldab
-        if getattr(h, "primary", None) is not None:     # shared pair: the primary's factors, read once
-            tot += ns * 32 * n
+        tot += ns * 32 * n
+        if getattr(h, "primary", None) is not None:     # shared pair: the primary's factors
             continue
-        tot += ns * (ef * (ldab * n + 2 * r * n + r * r) + 4 * n + 32 * n)
+        ops = ctypes.c_uint64()
+        call("cng_banded_operation_bytes", h.h, int(dev.precision == "fp32"), ctypes.byref(ops))
+        if ops.value:
+            tot += int(ops.value) + ns * 2 * n
+        else:
+            tot += ns * (ef * (ldab * n + 2 * r * n + r * r) + 4 * n)
     return tot
 
 
@@ -159,6 +166,9 @@ TRAFFIC_PER_SYSTEM = {
                                                    "profiles/k_solve_compact_multi_channel64x129x64_fp64.md"),
     ("channel", "fp64", "k_solve_window_multi"): ((177.924352 + 15.470848) * 1e6 / 1985,
                                                   "profiles/k_solve_window_multi_lanes8_channel64x129x64_fp64.md"),
+    # the scheduled solve: the operations a system's sweeps need, in slots of 16 or 8
+    ("channel", "fp64", "k_solve_flow"): ((113.845248 + 3.622912) * 1e6 / 1985, "profiles/k_solve_flow.md"),
+    ("channel", "fp32", "k_solve_flow"): ((81.797888 + 2.779136) * 1e6 / 1985, "profiles/k_solve_flow.md"),
     # the FP32 form solves in two groups: the captured launch is the group of 1024 paired systems
     ("channel", "fp32", "k_solve_compact_multi"): ((47.700736 + 0.423936) * 1e6 / 1024,
                                                    "profiles/k_solve_compact_multi_channel64x129x64_fp32.md"),

@@ -62,6 +62,7 @@ _SIGS = {
     "cng_banded_schedules": [P, P, P, P],
     "cng_banded_set_schedule": [P, c_int],
     "cng_banded_set_schedule_all": [c_int, P, c_int],
+    "cng_banded_operation_bytes": [P, c_int, P],
     "cng_banded_solve_fp32": [P, P, P, c_int, P],
     "cng_poly_residual": [c_int, c_int, P, P, P, P, P, c_int, c_double, c_double, P, P, P, P],
     "cng_twiddle_table": [c_int, c_int, P],

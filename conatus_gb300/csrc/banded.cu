@@ -1309,6 +1309,14 @@ int cng_banded_info(const cng_banded* hh, int32_t* dims, double* stats) {
     })
 }
 
+int cng_banded_operation_bytes(const cng_banded* hh, int fp32, uint64_t* bytes) {
+    CNG_TRY({
+        const Banded* h = as_banded(hh);
+        if (!bytes) throw InvalidArgument("null output");
+        *bytes = h->flow ? h->flow->used[fp32 ? 1 : 0] : 0;
+    })
+}
+
 int cng_banded_capacitance_cond(const cng_banded* hh, double* cond_host) {
     CNG_TRY({
         const Banded* h = as_banded(hh);

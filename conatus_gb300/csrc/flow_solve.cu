@@ -485,6 +485,10 @@ struct FlowBuild {
             if (total) k_flow_demote<<<blocks((size_t)total), 256, 0, st>>>(f->data[0], f->data[1], total, per);
             CNG_LAUNCH("k_flow_demote");
         }
+        for (int k = 0; k < B; ++k) {
+            f->used[0] += (size_t)h[k] * chunk;
+            if (s.fp32) f->used[1] += (size_t)h[k] * flow_chunk(f->ncr, 4);
+        }
         CNG_CUDA(cudaMemcpyAsync(f->nchunk, h.data(), sizeof(int) * B, cudaMemcpyHostToDevice, st));
         CNG_CUDA(cudaStreamSynchronize(st));
     }

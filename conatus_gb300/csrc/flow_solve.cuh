@@ -37,6 +37,7 @@ struct FlowForm {
     int ncr = 0;                         // right-hand sides of a factor: components x (system, partner)
     int chunks = 0;                      // largest number of chunks of operations of a system
     size_t sb[2] = {0, 0};               // bytes of a system: FP64, FP32
+    size_t used[2] = {0, 0};             // bytes that a solve of every system reads of them
     unsigned char* data[2] = {nullptr, nullptr};
     int* nchunk = nullptr;               // per system
     unsigned short* row = nullptr;       // [batch][n]: the name of each row

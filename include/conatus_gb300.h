@@ -183,6 +183,9 @@ int cng_banded_schedules(int32_t* count, int32_t* chunk, int32_t* stages, int32_
 int cng_banded_set_schedule(cng_banded* h, int sched);
 /* The same for nh handles, all or none of them; what they need is made side by side. */
 int cng_banded_set_schedule_all(int nh, cng_banded* const* h, int sched);
+/* Bytes of operations (FP64 or their FP32 copies) that a scheduled solve of the whole batch reads; 0 where the
+ * handle has none. */
+int cng_banded_operation_bytes(const cng_banded* h, int fp32, uint64_t* bytes);
 
 /* Mixed precision: keep FP32 (complex64) copies of the FP64 factors (allocates; refreshed by
  * refactor_shared). No reference counterpart: the FP32 + FP64-refinement form of the solve. */
