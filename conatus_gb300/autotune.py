@@ -104,10 +104,10 @@ def choose_solve(dev, key, fs, stream=None) -> dict:
     """The schedule of a new factor set: the scheduled solve where the systems take it, else the fastest of
     the others (``tune_solve``; so is every schedule of a problem that opts into the partitioned solve). Returns {schedule: ms per solve, or None where nothing was timed}.
 
-    The scheduled solve was the fastest candidate on every configuration: RB 256x64 0.036 ms against 0.161
-    for the next, channel 192x129x192 0.65 against 2.46 (FP32 form 1.33 against 2.11), Burgers 0.013
-    against 0.068, the RB ensembles 1.6x. Timing the others as well took 222 ms of a
-    new problem's first factorization there (16 candidates, four solves each), and ties between schedules
+    The scheduled solve was the fastest candidate on every configuration (a solve with its launch, as timed
+    here): RB 256x64 0.036 ms against 0.163 for the next, channel 192x129x192 0.66 against 2.46 (FP32 form
+    1.33 against 2.11), Burgers 0.024 against 0.070, the RB ensembles 1.6x. Timing the others as well took 222 ms
+    of a new problem's first factorization there (16 candidates, four solves each), and ties between schedules
     19 and 20 changed the bits from run to run."""
     sig = _signature(dev, fs)
     # a problem that opts into the partitioned solve (FP64 only) has it timed beside all the others

@@ -199,9 +199,10 @@ __device__ __forceinline__ void stage_ct(const c2<R>* __restrict__ a, c2<R>* __r
         // early stages (short runs of Ns consecutive outputs): the sequence index fastest across
         // the threads, so the stride-RAD writes of neighbouring threads fall in rows LS apart (LS
         // odd: other banks) instead of Ns RAD elements apart in one row (a few banks for all).
-        // Measured on the channel's F: the first stage in both precisions (FP32 2.40 -> 2.20 ms),
-        // the twiddled early stages in FP64 only (FP64 15.29 -> 14.94 ms; FP32 lost 0.07 ms: its
-        // twiddles are then loaded per butterfly instead of once per thread)
+        // The first stage in both precisions (the channel's FP32 F 2.40 -> 2.20 ms). The twiddled early
+        // stages in FP64 only, where the butterflies cost more than the twiddles that are then loaded for
+        // each (FP32 lost 0.07 ms by that); FP64 is left to Chebyshev columns without a Fourier
+        // direction and to FP64 ensembles, a column or a member to a block
         if ((B & (B - 1)) == 0) {
             const int sh = __ffs(B) - 1;
             for (int q = threadIdx.x; q < Lr * B; q += nt) {

@@ -4,10 +4,11 @@
 // and SM), while it does 58 64-bit integer additions and 4.3 64 x 64-bit fixed-point products per
 // clock and SM. An FFT is mostly additions, and each of its outputs is a sum over one column, so its
 // FP64 error is absolute in the column's norm: block floating point in 64-bit integers with one
-// exponent per column loses nothing. A column is scaled so that the sum of its entries' magnitudes,
-// which bounds every intermediate sum, is below 2^61: its values keep up to 61 bits. Measured
-// against 128-bit transforms, the error is below the FP64 transforms' for flat and for decaying
-// spectra (tests/test_fixed_transforms*.py).
+// exponent per column loses nothing against the column's norm. A column is scaled so that the sum of its
+// entries' magnitudes, which bounds every intermediate sum, is below 2^61: its largest entries keep up to 61
+// bits (about 53 in flat columns of 288 points, the least), the smaller ones fewer by their size. Measured
+// against 128-bit transforms, the error relative to the norm is below the FP64 transforms' for flat and
+// for decaying spectra (tests/test_fixed_transforms*.py).
 //
 // Products being the expensive part (13 additions each), the transforms are built for few of them:
 // L = 2^a 3^b 5^c is split by the prime-factor map (Good 1958, Thomas 1963) into blocks with no

@@ -21,7 +21,9 @@
 // complex update takes four.
 //
 // What bounds it: few systems, the chain of a slot (a shared-memory read, a fused multiply-add of 64
-// cycles, a write: 115 cycles); many, the FP64 unit (one warp instruction per 19 cycles and SM).
+// cycles, a write, two warp barriers: 140 cycles, from RB 256 x 64's 25.3 us for 354 slots and Burgers' 12.2 us
+// for 160 at 2.07 GHz, 2800 cycles beside the slots); many, the FP64 unit (channel 192 x 129 x 192: 657 us, a
+// slot per 23 cycles and SM, of which the unit takes 16).
 #include "flow_solve.cuh"
 
 #include <algorithm>

@@ -9,7 +9,14 @@
 
 namespace cng {
 
-// the most bytes of operations of a system per column; more are refused (memory.py plans them)
+// The most bytes of operations of a system per column; more are refused (memory.py plans them). A slot takes
+// 384 bytes with one right-hand side per factor, 192 with two, 96 with four (all its operations, used or
+// not), so this is a limit on slots: 1.04 a column for real systems, 2.08 for complex ones, 4.2 for shared pairs.
+// It is set by memory: what the planner counts for the steps' systems stays below the compact streams (about 790
+// bytes a column on the channel), and they fit it (slots a column: singles 0.9, Burgers 1.2, RB 1.35, the
+// channel's pairs 1.9). It is not where the time crosses: a real band that couples both parities takes 2 slots
+// a column and is refused from n of about 70 on, though its operations (700 bytes a column, its band 24) would
+// solve 31 systems of n = 200 in 26 us where the band kernel takes 69, and 2048 in 69 where it takes 123.
 constexpr int kFlowColumnBytes = 400;
 
 struct FlowSource {                      // the factored handle's arrays (banded.cu)

@@ -997,9 +997,9 @@ void complexify_kernel_launch(const R* in, void* out, long long n, cudaStream_t 
 template <class R>
 static void set_smem_attr(const void* fn) { ensure_smem_attr(fn, (int)kFftSmemMax); }
 
-// Sequences per block of the shared-memory transforms: at most 8 in FP32 and 4 in FP64 (measured
-// on the channel's F: fewer sequences per block, more blocks per SM; 16 was 6 % slower in FP32 and
-// 12 % in FP64, where the FP64 pipe is the bound and occupancy hides its latency).
+// Sequences per block of the shared-memory transforms: at most 8 in FP32 (measured on the channel's F:
+// fewer sequences per block, more blocks per SM; 16 was 6 % slower) and 4 in FP64, which is left to a
+// Chebyshev column per field of problems without a Fourier direction.
 constexpr int kMaxSeq32 = 8, kMaxSeq64 = 4;
 template <class R>
 static int pick_B(int L, int extra_per_col, int maxB) {
